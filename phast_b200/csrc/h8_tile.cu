@@ -49,6 +49,15 @@ __device__ __forceinline__ void cp_async_word(T* smem, const T* gmem) {
   const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(s), "l"(gmem), "n"(sizeof(T)) : "memory");
 }
+// One word, or zero where `live` is false (the source is then not read).
+template <typename T>
+__device__ __forceinline__ void cp_async_word_or_zero(T* smem, const T* gmem, bool live) {
+  static_assert(sizeof(T) == 4 || sizeof(T) == 8, "cp.async copies 4, 8 or 16 bytes");
+  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
+  const unsigned n = live ? (unsigned)sizeof(T) : 0u;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(s), "l"(gmem), "n"(sizeof(T)), "r"(n)
+               : "memory");
+}
 __device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 __device__ __forceinline__ unsigned long long global_ns() {
@@ -139,57 +148,27 @@ __device__ __forceinline__ void load_chunks(const unsigned char* base, int n, in
   }
 }
 
-// Node layer kn of the brick with its one-node halo, (ox+2)(oy+2) nodes, is
-// staged in two steps so the global loads of layer k+2 are in flight while
-// layer k's elements are computed: stage_load reads a thread's (at most two)
-// nodes into registers, stage_store writes them to buf[4][nt] (fields ux, uy,
-// uz, d).  Nodes outside a non-periodic grid read as zero.
+// A thread's (at most two) nodes of a layer, in registers (the wrapped halo nodes
+// that TMA staging patches).
 template <typename T>
 struct Staged {
   T v[2][4];
 };
 
-template <typename T>
-__device__ __forceinline__ void stage_load(const VoxGeom& g, const T* __restrict__ x, const T* __restrict__ d,
-                                           int i0, int j0, int kn, int ntx, int nt, Staged<T>& r) {
-  const int gk = wrap_node(kn, g.nz, g.rz, g.pz);
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int t = threadIdx.x + h * blockDim.x;
-    T u0 = T(0), u1 = T(0), u2 = T(0), dd = T(0);
-    if (t < nt && gk >= 0) {
-      const int a = t % ntx, b = t / ntx;
-      const int gi = wrap_node(i0 - 1 + a, g.nx, g.rx, g.px);
-      const int gj = wrap_node(j0 - 1 + b, g.ny, g.ry, g.py);
-      if (gi >= 0 && gj >= 0) {
-        const size_t n = (size_t)gi + (size_t)g.rx * ((size_t)gj + (size_t)g.ry * gk);
-        u0 = __ldg(x + 3 * n);
-        u1 = __ldg(x + 3 * n + 1);
-        u2 = __ldg(x + 3 * n + 2);
-        if (d) dd = __ldg(d + n);
-      }
-    }
-    r.v[h][0] = u0;
-    r.v[h][1] = u1;
-    r.v[h][2] = u2;
-    r.v[h][3] = dd;
-  }
+__device__ __forceinline__ void get4(const float* p, float (&v)[4]) {
+  const float4 q = *reinterpret_cast<const float4*>(p);
+  v[0] = q.x;
+  v[1] = q.y;
+  v[2] = q.z;
+  v[3] = q.w;
 }
-
-template <typename T>
-__device__ __forceinline__ void stage_store(int nt, const Staged<T>& r, T* buf) {
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int t = threadIdx.x + h * blockDim.x;
-    if (t < nt) {
-      buf[t] = r.v[h][0];
-      buf[nt + t] = r.v[h][1];
-      buf[2 * nt + t] = r.v[h][2];
-      buf[3 * nt + t] = r.v[h][3];
-    }
-  }
+__device__ __forceinline__ void get4(const double* p, double (&v)[4]) {
+  const double2 q = reinterpret_cast<const double2*>(p)[0], r = reinterpret_cast<const double2*>(p)[1];
+  v[0] = q.x;
+  v[1] = q.y;
+  v[2] = r.x;
+  v[3] = r.y;
 }
-
 
 template <typename T>
 __device__ __forceinline__ void ip2(T a0, T a1, T c1, T c2, T& q0, T& q1) {
@@ -265,14 +244,33 @@ __device__ __forceinline__ void grad_k_t(const T (&Px)[2][2], const T (&Py)[2][2
   }
 }
 
+// One node layer as an element sees it: the four corner values of u~ in the Haar basis of the
+// face (x difference X, y difference Y, mixed difference XY; the sum M as four times the first
+// corner's value V plus differences R, so that only differences of nodal values are ever rounded),
+// and 1 - d at the face's four Gauss positions o[qx + 2 qy] (interpolated in x and y).
 template <typename T>
-__device__ __forceinline__ T g_deg(T kappa, T d) {
-  const T o = T(1) - d;
-  return (T(1) - kappa) * o * o + kappa;
-}
+struct Face {
+  T V[3], R[3], X[3], Y[3], XY[3];
+  T o[4];
+};
+
+// The element's share of a node layer's forces, in the same Haar basis.
+template <typename T>
+struct FaceForce {
+  T M[3], X[3], Y[3], XY[3];
+};
 
 }  // namespace
 
+// What bounds it: instruction issue.  An element costs about 490 FP instructions: its strains and forces are
+// evaluated in the Haar (modal) basis of its eight corners, where a gradient component at the Gauss points is two
+// butterflies of scaled modes, and each face's modes and force modes are formed once and shared by the two
+// elements that meet there, through registers, since a thread marches up its element column.  The nodal form
+// before it (interpolating every face difference per element, lower and upper corner forces through shared
+// memory) issued 1 250.  Node layers are copied global -> shared with cp.async two layers ahead (no staging
+// registers), and in-plane offsets are formed once per brick.  Measured per action, this and the nodal form:
+// 64^3 FP32 24.7 / 29.3 us, FP64 32.9 / 51.8; 192^3 FP32 284 / 450, FP64 511 / 804; 97 x 83 x 110 FP64 84 / 144.
+//
 // One launch = every brick of the grid (persistent blocks).  COEF selects the
 // element coefficients (material slot + g(d), isotropic or general Voigt, or
 // per-Gauss-point moduli of a multigrid coarse level); MODE selects the node
@@ -312,7 +310,7 @@ __device__ __forceinline__ void tile_body(const TileArgs<T>& a, const VoxMat<T>&
           : smem_raw;
   const int W = tma_wx<T>(ox), Wd = tma_wd<T>(ox);
   const size_t xbb = tma_xbytes<T>(ox, oy), dbb = tma_dbytes<T>(ox, oy);
-  T* nb = reinterpret_cast<T*>(sbase);  // [3 buffers][4 fields][nt] (without TMA)
+  T* nb = reinterpret_cast<T*>(sbase);  // [3 buffers][nt][4 fields] (without TMA)
   size_t off_face = 0, off_qp = 0, off_cheb = 0;
   if (TMA) {
     tile_layout_tma<T>(ox, oy, COEF == kCoefQP, CHEB, &off_face, &off_qp, &off_cheb);
@@ -320,13 +318,11 @@ __device__ __forceinline__ void tile_body(const TileArgs<T>& a, const VoxMat<T>&
     tile_layout<T>(ox, oy, COEF == kCoefQP, CHEB, &off_qp, &off_cheb);
     off_face = sizeof(T) * 12 * (size_t)nt;
   }
-  T* FL = reinterpret_cast<T*>(sbase + off_face);  // [4 corners][3 comps][exy], lower face (oz = 0)
-  T* FU = FL + 12 * exy;                           // upper face (oz = 1)
+  T* FC = reinterpret_cast<T*>(sbase + off_face);  // corner forces of one node layer, [4 corners][3 comps][exy]
   // staged by cp.async, two buffers each: kCoefQP (lam_q, mu_q) of this thread's
   // element one element layer ahead, chunk-major [2][chunks][exy]; kModeCheb
   // (res, invd, xs) of this thread's owned node, [2][9][ox*oy], copied while the
   // layer's elements are computed
-  constexpr bool STAGE = COEF == kCoefQP || CHEB;
   constexpr int kQChunks = kStageQP * (int)sizeof(T) / 16;
   unsigned char* QS = sbase + off_qp;
   T* CS = reinterpret_cast<T*>(sbase + off_cheb);
@@ -347,12 +343,10 @@ __device__ __forceinline__ void tile_body(const TileArgs<T>& a, const VoxMat<T>&
   const int tid = threadIdx.x;
   const T w = T(g.w);
   const T c1 = T(a.c1), c2 = T(a.c2);
-  T E6[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
-  if (EROWS) {  // a Chebyshev step smooths the nodal block only (E rows masked)
-    const T* Ex = x + 3 * (size_t)g.n_red;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) E6[k] = __ldg(Ex + k);
-  }
+  // macro strain, read from shared memory where it is used (six registers fewer per thread); a Chebyshev
+  // step smooths the nodal block only (E rows masked).  The first barrier of the march orders the store.
+  __shared__ T E6[6];
+  if (EROWS && tid < 6) E6[tid] = __ldg(x + 3 * (size_t)g.n_red + tid);
   const int tiles_x = (g.rx + ox - 1) / ox, tiles_y = (g.ry + oy - 1) / oy;
   const int tiles_xy = tiles_x * tiles_y;
   const int n_tiles = tiles_xy * ((g.rz + kz - 1) / kz);
@@ -368,7 +362,39 @@ __device__ __forceinline__ void tile_body(const TileArgs<T>& a, const VoxMat<T>&
       if (c < 3) return reinterpret_cast<const T*>(sbase + (size_t)buf * xbb)[row * W + xr + 3 * col + c];
       return reinterpret_cast<const T*>(sbase + 3 * xbb + (size_t)buf * dbb)[row * Wd + dr + col];
     } else {
-      return nb[4 * nt * buf + c * nt + row * ntx + col];
+      return nb[4 * (nt * buf + row * ntx + col) + c];
+    }
+  };
+  // the upper or lower face of this thread's element from layer buffer `buf`
+  auto load_face = [&](int buf, Face<T>& f) {
+    T v[4][4];  // [corner][ux, uy, uz, d]
+#pragma unroll
+    for (int L = 0; L < 4; ++L) {
+      const int row = eb + (L >> 1), col = ea + (L & 1);
+      if constexpr (TMA) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) v[L][c] = nval(buf, c, row, col);
+        v[L][3] = use_d ? nval(buf, 3, row, col) : T(0);
+      } else {
+        get4(nb + 4 * (nt * buf + row * ntx + col), v[L]);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const T d0 = v[1][c] - v[0][c], d1 = v[3][c] - v[2][c];
+      const T e0 = v[2][c] - v[0][c], e1 = v[3][c] - v[1][c];
+      f.V[c] = v[0][c];
+      f.X[c] = d0 + d1;
+      f.Y[c] = e0 + e1;
+      f.XY[c] = d1 - d0;
+      f.R[c] = f.X[c] + T(2) * e0;
+    }
+    if (use_d) {
+      T a0, a1, b0, b1;
+      ip2(T(1) - v[0][3], T(1) - v[1][3], a.k.c1, a.k.c2, a0, a1);
+      ip2(T(1) - v[2][3], T(1) - v[3][3], a.k.c1, a.k.c2, b0, b1);
+      ip2(a0, b0, a.k.c1, a.k.c2, f.o[0], f.o[2]);
+      ip2(a1, b1, a.k.c1, a.k.c2, f.o[1], f.o[3]);
     }
   };
   // TMA: thread 0 issues the copies of node layer kn into buffer b
@@ -433,76 +459,101 @@ __device__ __forceinline__ void tile_body(const TileArgs<T>& a, const VoxMat<T>&
     }
   };
   double accd[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  // material slot of this thread's element in layer ke (0 outside the grid)
-  auto elem_slot = [&](int i0, int j0, int ke) -> int {
-    if (!SLOT || !is_elem) return 0;
-    const int gi = wrap_elem(i0 - 1 + ea, g.nx, g.px);
-    const int gj = wrap_elem(j0 - 1 + eb, g.ny, g.py);
-    const int gk = wrap_elem(ke, g.nz, g.pz);
-    if (gi < 0 || gj < 0 || gk < 0) return 0;
-    return __ldg(a.slot + (size_t)gi + (size_t)g.nx * ((size_t)gj + (size_t)g.ny * gk));
-  };
-  // fixed-dof bits (one per component) of this thread's owned node in layer kn
-  auto node_mask = [&](int i0, int j0, int kn) -> int {
-    if (!a.mask || !is_node || kn >= g.rz) return 0;
-    const int gi = i0 + ni, gj = j0 + nj;
-    if (gi >= g.rx || gj >= g.ry) return 0;
-    const size_t n = (size_t)gi + (size_t)g.rx * ((size_t)gj + (size_t)g.ry * kn);
-    return (__ldg(a.mask + 3 * n) ? 1 : 0) | (__ldg(a.mask + 3 * n + 1) ? 2 : 0) |
-           (__ldg(a.mask + 3 * n + 2) ? 4 : 0);
-  };
-  // Staging commit groups, in order: per step kk one Chebyshev group (node layer
-  // ke) then one moduli group (element layer ke + 1), each possibly empty, so the
-  // number of groups committed after any one of them is fixed.
-  // kCoefQP: copies element layer ke's (lam_q, mu_q) into buffer `buf`.
-  auto stage_qp = [&](int i0, int j0, int ke, int buf, bool live) {
-    if constexpr (STAGE) {
-      if (COEF == kCoefQP && live && q_async && is_elem) {
-        const int gi = wrap_elem(i0 - 1 + ea, g.nx, g.px);
-        const int gj = wrap_elem(j0 - 1 + eb, g.ny, g.py);
-        const int gk = wrap_elem(ke, g.nz, g.pz);
-        if (gi >= 0 && gj >= 0 && gk >= 0) {
-          const size_t e = (size_t)gi + (size_t)g.nx * ((size_t)gj + (size_t)g.ny * gk);
-          unsigned char* dst = QS + (size_t)buf * kQChunks * exy * 16;
-          stage_chunks(dst, exy, tid, 0, a.lam_q + 8 * e, kQChunks / 2);
-          stage_chunks(dst, exy, tid, kQChunks / 2, a.mu_q + 8 * e, kQChunks / 2);
-        }
-      }
-      cp_async_commit();
-    }
-  };
-  // kModeCheb: copies (res, invd, xs) of the owned node in node layer kn into buffer `buf`.
-  auto stage_cheb = [&](int i0, int j0, int kn, int buf, bool live) {
-    if constexpr (STAGE) {
-      const int gi = i0 + ni, gj = j0 + nj;
-      if (CHEB && live && is_node && gi < g.rx && gj < g.ry) {
-        const size_t n3 = 3 * ((size_t)gi + (size_t)g.rx * ((size_t)gj + (size_t)g.ry * kn));
-        T* dst = CS + (size_t)buf * 9 * oxy + tid;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          cp_async_word(dst + c * oxy, a.res + n3 + c);
-          cp_async_word(dst + (3 + c) * oxy, a.invd + n3 + c);
-          cp_async_word(dst + (6 + c) * oxy, a.xs + n3 + c);
-        }
-      }
-      cp_async_commit();
-    }
-  };
+  const size_t plane_n = (size_t)g.rx * g.ry, plane_e = (size_t)g.nx * g.ny;
 
   for (int tile = vb; tile < n_tiles; tile += vgrid) {
     const int tz = tile / tiles_xy, txy = tile - tz * tiles_xy;
     const int i0 = (txy % tiles_x) * ox, j0 = (txy / tiles_x) * oy;
     const int k0 = tz * kz, k1 = min(k0 + kz, g.rz);
+    // In-plane offsets of this thread's staged nodes, element and owned node, once per brick (-1: outside
+    // the grid or not this thread's); a layer then adds one uniform plane offset.
+    int so[2], eo = -1, no = -1;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int t = tid + h * blockDim.x;
+      so[h] = -1;
+      if (t < nt) {
+        const int gi = wrap_node(i0 - 1 + t % ntx, g.nx, g.rx, g.px);
+        const int gj = wrap_node(j0 - 1 + t / ntx, g.ny, g.ry, g.py);
+        if (gi >= 0 && gj >= 0) so[h] = gi + g.rx * gj;
+      }
+    }
+    if (is_elem) {
+      const int gi = wrap_elem(i0 - 1 + ea, g.nx, g.px);
+      const int gj = wrap_elem(j0 - 1 + eb, g.ny, g.py);
+      if (gi >= 0 && gj >= 0) eo = gi + g.nx * gj;
+    }
+    if (is_node && i0 + ni < g.rx && j0 + nj < g.ry) no = (i0 + ni) + g.rx * (j0 + nj);
+    const bool own_xy = ea >= 1 && eb >= 1 && i0 - 1 + ea < g.rx && j0 - 1 + eb < g.ry;
+    // cp.async of node layer kn into buffer b (zeros outside the grid)
+    auto stage_nodes = [&](int kn, int b) {
+      const int gk = wrap_node(kn, g.nz, g.rz, g.pz);
+      const T* xk = x + 3 * (plane_n * (size_t)(gk < 0 ? 0 : gk));
+      const T* dk = use_d ? d + plane_n * (size_t)(gk < 0 ? 0 : gk) : nullptr;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int t = tid + h * blockDim.x;
+        if (t < nt) {
+          const bool live = so[h] >= 0 && gk >= 0;
+          const int o = so[h] >= 0 ? so[h] : 0;
+          T* dst = nb + 4 * (nt * b + t);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) cp_async_word_or_zero(dst + c, xk + 3 * (size_t)o + c, live);
+          if (use_d) cp_async_word_or_zero(dst + 3, dk + o, live);
+        }
+      }
+    };
+    // material slot of this thread's element in layer ke (0 outside the grid)
+    auto elem_slot = [&](int ke) -> int {
+      const int gk = wrap_elem(ke, g.nz, g.pz);
+      return SLOT && eo >= 0 && gk >= 0 ? __ldg(a.slot + plane_e * gk + eo) : 0;
+    };
+    // fixed-dof bits (one per component) of this thread's owned node in layer kn
+    auto node_mask = [&](int kn) -> int {
+      if (!a.mask || no < 0 || kn >= g.rz) return 0;
+      const uint8_t* mp = a.mask + 3 * (plane_n * kn + no);
+      return (__ldg(mp) ? 1 : 0) | (__ldg(mp + 1) ? 2 : 0) | (__ldg(mp + 2) ? 4 : 0);
+    };
+    // kCoefQP: cp.async of element layer ke's (lam_q, mu_q) into buffer `buf`
+    auto stage_qp = [&](int ke, int buf) {
+      if constexpr (COEF == kCoefQP) {
+        const int gk = wrap_elem(ke, g.nz, g.pz);
+        if (q_async && eo >= 0 && gk >= 0) {
+          const size_t e = plane_e * gk + eo;
+          unsigned char* dst = QS + (size_t)buf * kQChunks * exy * 16;
+          stage_chunks(dst, exy, tid, 0, a.lam_q + 8 * e, kQChunks / 2);
+          stage_chunks(dst, exy, tid, kQChunks / 2, a.mu_q + 8 * e, kQChunks / 2);
+        }
+      }
+    };
+    // kModeCheb: cp.async of (res, invd, xs) of the owned node in node layer kn into buffer `buf`
+    auto stage_cheb = [&](int kn, int buf) {
+      if constexpr (CHEB) {
+        if (no >= 0) {
+          const size_t n3 = 3 * (plane_n * kn + no);
+          T* dst = CS + (size_t)buf * 9 * oxy + tid;
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            cp_async_word(dst + c * oxy, a.res + n3 + c);
+            cp_async_word(dst + (3 + c) * oxy, a.invd + n3 + c);
+            cp_async_word(dst + (6 + c) * oxy, a.xs + n3 + c);
+          }
+        }
+      }
+    };
     T tacc[8] = {T(0), T(0), T(0), T(0), T(0), T(0), T(0), T(0)};
-    T pend[3] = {T(0), T(0), T(0)};
+    Face<T> fl;         // lower face of this thread's element
+    FaceForce<T> pend;  // force of the element below on that face
+#pragma unroll
+    for (int c = 0; c < 3; ++c) pend.M[c] = pend.X[c] = pend.Y[c] = pend.XY[c] = T(0);
     Staged<T> pf;
     unsigned pf_on = 0;
+    __syncthreads();  // the previous tile's last node phase is done with the buffers
     if constexpr (TMA) {
       xs0 = floor_mult(3 * (i0 - 1), kA);
       xr = 3 * (i0 - 1) - xs0;
       ds0 = floor_mult(i0 - 1, kA);
       dr = (i0 - 1) - ds0;
-      __syncthreads();  // the previous tile's last node phase is done with the buffers
       tma_issue(i0, j0, k0 - 1, 0);
       tma_issue(i0, j0, k0, 1);
       wrap_load(i0, j0, k0 - 1, pf, pf_on);
@@ -510,216 +561,252 @@ __device__ __forceinline__ void tile_body(const TileArgs<T>& a, const VoxMat<T>&
       wrap_store(pf, pf_on, 0);
       wrap_load(i0, j0, k0, pf, pf_on);
     } else {
-      stage_load(g, x, d, i0, j0, k0 - 1, ntx, nt, pf);
-      __syncthreads();  // the previous tile's last node phase is done with the buffers
-      stage_store(nt, pf, nb);
-      stage_load(g, x, d, i0, j0, k0, ntx, nt, pf);
+      stage_nodes(k0 - 1, 0);
+      stage_nodes(k0, 1);
     }
-    int sl_next = elem_slot(i0, j0, k0 - 1);
-    stage_qp(i0, j0, k0 - 1, 0, true);
-    int mk_next = node_mask(i0, j0, k0), mk_cur = 0;
+    int sl_next = elem_slot(k0 - 1);
+    stage_qp(k0 - 1, 0);
+    cp_async_commit();
+    int mk_next = node_mask(k0), mk_cur = 0;
     const int K = k1 - k0;
+    // Commit groups of a step: the Chebyshev data of node layer ke, then the moduli of element layer ke + 1
+    // with node layer ke + 2.
     for (int kk = 0; kk <= K; ++kk) {
       const int ke = k0 - 1 + kk;  // element layer of this step
       const int ib0 = kk % 3, ib1 = (kk + 1) % 3;
       if constexpr (TMA) {
         tma_wait(ib1);  // node layer ke + 1
         wrap_store(pf, pf_on, ib1);
-      } else {
-        stage_store(nt, pf, nb + 4 * nt * ib1);  // node layer ke + 1
       }
+      cp_async_wait<0>();  // node layer ke + 1 and the moduli of element layer ke have landed
       const int sl = sl_next;
-      if (kk < K) {
-        if constexpr (TMA)
-          wrap_load(i0, j0, ke + 2, pf, pf_on);
-        else
-          stage_load(g, x, d, i0, j0, ke + 2, ntx, nt, pf);
-        sl_next = elem_slot(i0, j0, ke + 1);
-      }
-      if constexpr (STAGE) {
-        stage_cheb(i0, j0, ke, kk & 1, kk >= 1);
-        stage_qp(i0, j0, ke + 1, (kk + 1) & 1, kk < K);
-        cp_async_wait<2>();  // this thread's moduli of element layer ke have landed
-      }
       if (kk >= 1) {
         mk_cur = mk_next;
-        if (kk < K) mk_next = node_mask(i0, j0, ke + 1);
+        if (kk < K) mk_next = node_mask(ke + 1);
       }
       __syncthreads();
       // every thread is done with buffer (kk + 2) % 3 (node layer ke - 1): refill it with layer ke + 2
-      if (kk < K) tma_issue(i0, j0, ke + 2, (kk + 2) % 3);
+      if constexpr (CHEB) {
+        if (kk >= 1) stage_cheb(ke, kk & 1);
+        cp_async_commit();
+      }
+      if (kk < K) {
+        if constexpr (TMA) {
+          tma_issue(i0, j0, ke + 2, (kk + 2) % 3);
+          wrap_load(i0, j0, ke + 2, pf, pf_on);
+        } else {
+          stage_nodes(ke + 2, (kk + 2) % 3);
+        }
+        stage_qp(ke + 1, (kk + 1) & 1);
+        sl_next = elem_slot(ke + 1);
+      }
+      cp_async_commit();
       // ---- element phase: one element of the (ox+1) x (oy+1) tile per thread
       if (is_elem) {
-        const int gi = wrap_elem(i0 - 1 + ea, g.nx, g.px);
-        const int gj = wrap_elem(j0 - 1 + eb, g.ny, g.py);
+        if (kk == 0) load_face(ib0, fl);
+        Face<T> fu;
+        load_face(ib1, fu);
         const int gk = wrap_elem(ke, g.nz, g.pz);
-        T f[3][8];
-        if (gi >= 0 && gj >= 0 && gk >= 0) {
-          const size_t e = (size_t)gi + (size_t)g.nx * ((size_t)gj + (size_t)g.ny * gk);
-          const bool own = ea >= 1 && eb >= 1 && kk >= 1 && i0 - 1 + ea < g.rx && j0 - 1 + eb < g.ry;
-          T gv[8];
-          if (SLOT) {
-            if (a.gq) {
+        // lo: the column's whole force on node layer ke, the upper face of the element below (pend) plus
+        // the lower face of this one
+        FaceForce<T> lo = pend;
 #pragma unroll
-              for (int q = 0; q < 8; ++q) gv[q] = __ldg(a.gq + 8 * e + q);
-            } else if (d) {
-              T dd[8], dq[8];
-#pragma unroll
-              for (int L = 0; L < 8; ++L) dd[L] = nval((L & 4) ? ib1 : ib0, 3, eb + ((L >> 1) & 1), ea + (L & 1));
-              interp_sf(dd, dq);
-#pragma unroll
-              for (int q = 0; q < 8; ++q) gv[q] = g_deg(m.kappa, dq[q]);
-            } else {
-#pragma unroll
-              for (int q = 0; q < 8; ++q) gv[q] = T(1);
-            }
-          }
-          T D[3][3][2][2];
+        for (int c = 0; c < 3; ++c) pend.M[c] = pend.X[c] = pend.Y[c] = pend.XY[c] = T(0);
+        if (eo >= 0 && gk >= 0) {
+          const size_t e = plane_e * gk + eo;
+          const bool own = own_xy && kk >= 1;
+          const TileK<T>& k = a.k;
+          // z modes of the element: sums (X, Y, XY) and differences (Mz, Xz, Yz, XYz) of the two faces
+          T X[3], Y[3], XY[3], Mz[3], Xz[3], Yz[3], XYz[3];
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
-            T u[8];
-#pragma unroll
-            for (int L = 0; L < 8; ++L) u[L] = nval((L & 4) ? ib1 : ib0, c, eb + ((L >> 1) & 1), ea + (L & 1));
-            grad_k(u, a.k, D[c][0], D[c][1], D[c][2]);
+            X[c] = fl.X[c] + fu.X[c];
+            Y[c] = fl.Y[c] + fu.Y[c];
+            XY[c] = fl.XY[c] + fu.XY[c];
+            Mz[c] = T(4) * (fu.V[c] - fl.V[c]) + (fu.R[c] - fl.R[c]);
+            Xz[c] = fu.X[c] - fl.X[c];
+            Yz[c] = fu.Y[c] - fl.Y[c];
+            XYz[c] = fu.XY[c] - fl.XY[c];
           }
-          if (EROWS) {
-            // the macro strain enters each strain component once: fold it into
-            // the gradient term that component starts from
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-              for (int j = 0; j < 2; ++j) {
-                D[0][0][i][j] += E6[0];
-                D[1][1][i][j] += E6[1];
-                D[2][2][i][j] += E6[2];
-                D[1][2][i][j] += E6[3];
-                D[0][2][i][j] += E6[4];
-                D[0][1][i][j] += E6[5];
-              }
-          }
-          T P[3][3][2][2];
+          // d u_c / dz at [qy][qx]; the macro strain enters each strain component once, in the gradient
+          // term that component starts from
+          T Dz[3][2][2], Pz[3][2][2];
 #pragma unroll
           for (int c = 0; c < 3; ++c)
 #pragma unroll
-            for (int b = 0; b < 3; ++b)
+            for (int qx = 0; qx < 2; ++qx) {
+              const T sx = qx ? k.g : -k.g;
+              const T A = Mz[c] + sx * Xz[c], B = Yz[c] + sx * XYz[c];
+              const T t = k.az * A + (EROWS ? (c == 0 ? E6[4] : (c == 1 ? E6[3] : E6[2])) : T(0));
+              Dz[c][0][qx] = t - k.bz * B;
+              Dz[c][1][qx] = t + k.bz * B;
+            }
+          // coefficients of the material: lam and mu times the quadrature weight
+          const T lw = COEF == kCoefIso ? m.lam[sl] * w : T(0), mw = COEF == kCoefIso ? m.mu[sl] * w : T(0);
+          const T kap = T(m.kappa), okap = T(1) - kap;
+          // sums over the Gauss points of each half (qz = 0, 1) for the transposed gradient
+          T Sx[3][2], Sy[3][2], Sxy[3][2];
 #pragma unroll
-              for (int i = 0; i < 2; ++i)
+          for (int qz = 0; qz < 2; ++qz) {
+            const T sz = qz ? k.g : -k.g;
+            T Dx[3][2], Dy[3][2];  // [qy], [qx]
 #pragma unroll
-                for (int j = 0; j < 2; ++j) P[c][b][i][j] = T(0);
-          // w * g_q * sigma_q at the eight Gauss points, summed into the P terms
-          auto qp_loop = [&](auto stress) {
+            for (int c = 0; c < 3; ++c) {
+              const T Ax = X[c] + sz * Xz[c], Ay = Y[c] + sz * Yz[c], B = XY[c] + sz * XYz[c];
+              const T tx = k.ax * Ax + (EROWS && c == 0 ? E6[0] : T(0));
+              const T ty = k.ay * Ay + (EROWS && c == 0 ? E6[5] : (EROWS && c == 1 ? E6[1] : T(0)));
+              Dx[c][0] = tx - k.bx * B;
+              Dx[c][1] = tx + k.bx * B;
+              Dy[c][0] = ty - k.by * B;
+              Dy[c][1] = ty + k.by * B;
+            }
+            // degradation (and, on coarse levels, the moduli) of the half's four Gauss points
+            T gv[4], lm[8];
+            if (SLOT) {
+              if (a.gq) {
 #pragma unroll
-            for (int qz = 0; qz < 2; ++qz)
+                for (int q = 0; q < 4; ++q) gv[q] = __ldg(a.gq + 8 * e + 4 * qz + q);
+              } else if (d) {
 #pragma unroll
-              for (int qy = 0; qy < 2; ++qy)
-#pragma unroll
-                for (int qx = 0; qx < 2; ++qx) {
-                  T ep[6];
-                  ep[0] = D[0][0][qz][qy];
-                  ep[1] = D[1][1][qz][qx];
-                  ep[2] = D[2][2][qy][qx];
-                  ep[3] = D[1][2][qy][qx] + D[2][1][qz][qx];
-                  ep[4] = D[0][2][qy][qx] + D[2][0][qz][qy];
-                  ep[5] = D[0][1][qz][qx] + D[1][0][qz][qy];
-                  T sg[6];
-                  stress(ep, qx + 2 * qy + 4 * qz, sg);
-                  if (ENERGY && own) {
-#pragma unroll
-                    for (int k = 0; k < 6; ++k) tacc[kOutEnergy] += T(0.5) * sg[k] * ep[k];
-                  }
-                  P[0][0][qz][qy] += sg[0];
-                  P[0][1][qz][qx] += sg[5];
-                  P[0][2][qy][qx] += sg[4];
-                  P[1][0][qz][qy] += sg[5];
-                  P[1][1][qz][qx] += sg[1];
-                  P[1][2][qy][qx] += sg[3];
-                  P[2][0][qz][qy] += sg[4];
-                  P[2][1][qz][qx] += sg[3];
-                  P[2][2][qy][qx] += sg[2];
+                for (int q = 0; q < 4; ++q) {
+                  const T o = qz ? k.c2 * fl.o[q] + k.c1 * fu.o[q] : k.c1 * fl.o[q] + k.c2 * fu.o[q];
+                  gv[q] = okap * (o * o) + kap;
                 }
-          };
-          auto iso_stress = [&](const T* ep, T lg, T mg, T* sg) {
-            const T mg2 = mg + mg;
-            const T lt = lg * (ep[0] + ep[1] + ep[2]);
-            sg[0] = mg2 * ep[0] + lt;
-            sg[1] = mg2 * ep[1] + lt;
-            sg[2] = mg2 * ep[2] + lt;
-            sg[3] = mg * ep[3];
-            sg[4] = mg * ep[4];
-            sg[5] = mg * ep[5];
-          };
-          if constexpr (COEF == kCoefIso) {
-            const T lw = m.lam[sl] * w, mw = m.mu[sl] * w;
-            qp_loop([&](const T* ep, int q, T* sg) { iso_stress(ep, lw * gv[q], mw * gv[q], sg); });
-          } else if constexpr (COEF == kCoefAniso) {
-            qp_loop([&](const T* ep, int q, T* sg) {
-              voigt_stress(m, sl, ep, sg);
-              const T gw = gv[q] * w;
+              } else {
 #pragma unroll
-              for (int k = 0; k < 6; ++k) sg[k] *= gw;
-            });
-          } else {
-            T lm[kStageQP];  // lam_q[0..7], mu_q[0..7]
-            if (q_async) {
-              load_chunks<T, kStageQP>(QS + (size_t)(kk & 1) * kQChunks * exy * 16, exy, tid, lm);
+                for (int q = 0; q < 4; ++q) gv[q] = T(1);
+              }
+            } else if (q_async) {
+              // chunks of the half: lam_q at qz * n, mu_q after all of lam_q
+              constexpr int nc = kQChunks / 4;
+              const unsigned char* qs = QS + (size_t)(kk & 1) * kQChunks * exy * 16;
+              T l4[4], m4[4];
+              load_chunks<T, 4>(qs + (size_t)qz * nc * exy * 16, exy, tid, l4);
+              load_chunks<T, 4>(qs + (size_t)(2 + qz) * nc * exy * 16, exy, tid, m4);
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                lm[q] = l4[q];
+                lm[4 + q] = m4[q];
+              }
             } else {
 #pragma unroll
-              for (int q = 0; q < 8; ++q) {
-                lm[q] = __ldg(a.lam_q + 8 * e + q);
-                lm[8 + q] = __ldg(a.mu_q + 8 * e + q);
+              for (int q = 0; q < 4; ++q) {
+                lm[q] = __ldg(a.lam_q + 8 * e + 4 * qz + q);
+                lm[4 + q] = __ldg(a.mu_q + 8 * e + 4 * qz + q);
               }
             }
-            qp_loop([&](const T* ep, int q, T* sg) { iso_stress(ep, lm[q] * w, lm[8 + q] * w, sg); });
-          }
-          if (EROWS && own) {
+            T Px[3][2], Py[3][2];
 #pragma unroll
-            for (int i = 0; i < 2; ++i)
+            for (int qy = 0; qy < 2; ++qy)
 #pragma unroll
-              for (int j = 0; j < 2; ++j) {
-                tacc[0] += P[0][0][i][j];
-                tacc[1] += P[1][1][i][j];
-                tacc[2] += P[2][2][i][j];
-                tacc[3] += P[1][2][i][j];
-                tacc[4] += P[0][2][i][j];
-                tacc[5] += P[0][1][i][j];
+              for (int qx = 0; qx < 2; ++qx) {
+                const int q = qx + 2 * qy;
+                T ep[6], sg[6];
+                ep[0] = Dx[0][qy];
+                ep[1] = Dy[1][qx];
+                ep[2] = Dz[2][qy][qx];
+                ep[3] = Dz[1][qy][qx] + Dy[2][qx];
+                ep[4] = Dz[0][qy][qx] + Dx[2][qy];
+                ep[5] = Dy[0][qx] + Dx[1][qy];
+                if constexpr (COEF == kCoefAniso) {
+                  voigt_stress(m, sl, ep, sg);
+                  const T gw = gv[q] * w;
+#pragma unroll
+                  for (int i = 0; i < 6; ++i) sg[i] *= gw;
+                } else {
+                  const T lg = COEF == kCoefIso ? lw * gv[q] : lm[q] * w;
+                  const T mg = COEF == kCoefIso ? mw * gv[q] : lm[4 + q] * w;
+                  const T mg2 = mg + mg;
+                  const T lt = lg * (ep[0] + ep[1] + ep[2]);
+                  sg[0] = mg2 * ep[0] + lt;
+                  sg[1] = mg2 * ep[1] + lt;
+                  sg[2] = mg2 * ep[2] + lt;
+                  sg[3] = mg * ep[3];
+                  sg[4] = mg * ep[4];
+                  sg[5] = mg * ep[5];
+                }
+                if (ENERGY && own) {
+#pragma unroll
+                  for (int i = 0; i < 6; ++i) tacc[kOutEnergy] += T(0.5) * sg[i] * ep[i];
+                }
+                // first contribution to a sum assigns, the others add
+                Px[0][qy] = qx == 0 ? sg[0] : Px[0][qy] + sg[0];
+                Px[1][qy] = qx == 0 ? sg[5] : Px[1][qy] + sg[5];
+                Px[2][qy] = qx == 0 ? sg[4] : Px[2][qy] + sg[4];
+                Py[0][qx] = qy == 0 ? sg[5] : Py[0][qx] + sg[5];
+                Py[1][qx] = qy == 0 ? sg[1] : Py[1][qx] + sg[1];
+                Py[2][qx] = qy == 0 ? sg[3] : Py[2][qx] + sg[3];
+                Pz[0][qy][qx] = qz == 0 ? sg[4] : Pz[0][qy][qx] + sg[4];
+                Pz[1][qy][qx] = qz == 0 ? sg[3] : Pz[1][qy][qx] + sg[3];
+                Pz[2][qy][qx] = qz == 0 ? sg[2] : Pz[2][qy][qx] + sg[2];
               }
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+              Sx[c][qz] = Px[c][0] + Px[c][1];
+              Sy[c][qz] = Py[c][0] + Py[c][1];
+              Sxy[c][qz] = k.ax * (Px[c][1] - Px[c][0]) + k.ay * (Py[c][1] - Py[c][0]);
+            }
           }
-#pragma unroll
-          for (int c = 0; c < 3; ++c) grad_k_t(P[c][0], P[c][1], P[c][2], a.k, f[c]);
-        } else {
-#pragma unroll
-          for (int c = 0; c < 3; ++c)
-#pragma unroll
-            for (int L = 0; L < 8; ++L) f[c][L] = T(0);
-        }
-#pragma unroll
-        for (int L = 0; L < 4; ++L)
+          // transposed gradient: the element's modal forces, split into its two faces
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
-            FL[(L * 3 + c) * exy + tid] = f[c][L];
-            FU[(L * 3 + c) * exy + tid] = f[c][L + 4];
+            const T p0 = Pz[c][0][0] + Pz[c][0][1], p1 = Pz[c][1][0] + Pz[c][1][1];
+            const T m0 = Pz[c][0][1] - Pz[c][0][0], m1 = Pz[c][1][1] - Pz[c][1][0];
+            const T T0 = p0 + p1, TY = p1 - p0, TX = m0 + m1, TXY = m1 - m0;
+            const T sx = Sx[c][0] + Sx[c][1], sy = Sy[c][0] + Sy[c][1];
+            if (EROWS && own) {
+              if (c == 0) {
+                tacc[0] += sx;
+                tacc[5] += sy;
+                tacc[4] += T0;
+              } else if (c == 1) {
+                tacc[1] += sy;
+                tacc[3] += T0;
+              } else {
+                tacc[2] += T0;
+              }
+            }
+            const T fX = k.ax * sx, fY = k.ay * sy, fXY = k.g * (Sxy[c][0] + Sxy[c][1]);
+            const T fM = k.az * T0;
+            const T fXz = k.bx * (Sx[c][1] - Sx[c][0]) + k.bz * TX;
+            const T fYz = k.by * (Sy[c][1] - Sy[c][0]) + k.bz * TY;
+            const T fXYz = k.g * (k.g * (Sxy[c][1] - Sxy[c][0]) + k.bz * TXY);
+            lo.M[c] -= fM;
+            lo.X[c] += fX - fXz;
+            lo.Y[c] += fY - fYz;
+            lo.XY[c] += fXY - fXYz;
+            pend.M[c] = fM;
+            pend.X[c] = fX + fXz;
+            pend.Y[c] = fY + fYz;
+            pend.XY[c] = fXY + fXYz;
           }
+        }
+        fl = fu;
+        if (kk >= 1) {
+          // corner forces on node layer ke: corner L = (x side, y side), component c at FC[(3 L + c) exy + tid]
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            const T mm = lo.M[c] - lo.Y[c], mp = lo.M[c] + lo.Y[c];
+            const T xm = lo.X[c] - lo.XY[c], xp = lo.X[c] + lo.XY[c];
+            FC[c * exy + tid] = mm - xm;
+            FC[(3 + c) * exy + tid] = mm + xm;
+            FC[(6 + c) * exy + tid] = mp - xp;
+            FC[(9 + c) * exy + tid] = mp + xp;
+          }
+        }
       }
+      if (kk == 0) continue;  // the first element layer only fills pend
       __syncthreads();
-      if constexpr (STAGE) cp_async_wait<1>();  // this thread's (res, invd, xs) of node layer ke
-      // ---- node phase: node layer ke = lower faces of this layer + upper faces of the previous
-      if (is_node) {
+      if constexpr (CHEB) cp_async_wait<1>();  // this thread's (res, invd, xs) of node layer ke
+      // ---- node phase: node layer ke, the four columns that meet at the node
+      if (no >= 0) {
         const int e11 = (ni + 1) + ex * (nj + 1), e01 = ni + ex * (nj + 1);
         const int e10 = (ni + 1) + ex * nj, e00 = ni + ex * nj;
-        T lo[3], up[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          lo[c] = FL[(0 * 3 + c) * exy + e11] + FL[(1 * 3 + c) * exy + e01] + FL[(2 * 3 + c) * exy + e10] +
-                  FL[(3 * 3 + c) * exy + e00];
-          up[c] = FU[(0 * 3 + c) * exy + e11] + FU[(1 * 3 + c) * exy + e01] + FU[(2 * 3 + c) * exy + e10] +
-                  FU[(3 * 3 + c) * exy + e00];
-        }
-        const int gi = i0 + ni, gj = j0 + nj;
-        if (kk >= 1 && gi < g.rx && gj < g.ry) {
-          const size_t n = (size_t)gi + (size_t)g.rx * ((size_t)gj + (size_t)g.ry * ke);
+        {
+          const size_t n = plane_n * ke + no;
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
-            T v = pend[c] + lo[c];
+            T v = (FC[c * exy + e11] + FC[(3 + c) * exy + e01]) + (FC[(6 + c) * exy + e10] + FC[(9 + c) * exy + e00]);
             if (mk_cur & (1 << c)) v = T(0);
             const size_t i = 3 * n + c;
             const T xin = nval(ib0, c, nj + 1, ni + 1);
@@ -736,8 +823,6 @@ __device__ __forceinline__ void tile_body(const TileArgs<T>& a, const VoxMat<T>&
             }
           }
         }
-#pragma unroll
-        for (int c = 0; c < 3; ++c) pend[c] = up[c];
       }
     }
     if (RED) {
@@ -792,14 +877,21 @@ __device__ __forceinline__ void tile_body(const TileArgs<T>& a, const VoxMat<T>&
   }
 }
 
+// Threads and resident blocks per SM the kernel is compiled for: 128 registers per thread in FP32 (about 16
+// warps per SM), 255 in FP64 (8 warps).  Fewer registers and more warps measured slower: FP32 at 96 registers
+// 30.4 against 25.9 us on 64^3, FP64 at two blocks of 160 threads 45.4 against 43.5 us (the spills).
+template <typename T, int OX, int OY>
+struct TileBounds {
+  static constexpr int threads = OX ? ((OX + 1) * (OY + 1) + 31) / 32 * 32 : kTileMaxThreads;
+  static constexpr int blocks = sizeof(T) == 4 ? 512 / threads : (threads > 128 ? 1 : 256 / threads);
+};
+
 template <typename T, int COEF, int MODE, int OX, int OY, bool TMA>
-__global__ void __launch_bounds__(kTileMaxThreads, sizeof(T) == 4 ? 2 : 1)
+__global__ void __launch_bounds__(TileBounds<T, OX, OY>::threads, TileBounds<T, OX, OY>::blocks)
     h8_tile_kernel(TileArgs<T> a, VoxMat<T> m, const __grid_constant__ CUtensorMap tmx,
                    const __grid_constant__ CUtensorMap tmd) {
   tile_body<T, COEF, MODE, OX, OY, TMA>(a, m, &tmx, &tmd, blockIdx.x, gridDim.x);
 }
-
-#include "h8_tile2.cuh"
 
 // ------------------------------------------------------------------ damage action
 
@@ -1186,10 +1278,10 @@ auto shape_key(const VoxGeom& g, int word, int cls) {
   return std::make_tuple(g.rx, g.ry, g.rz, g.px, g.py, g.pz, word, cls);
 }
 
-// Heuristic: among owned-node tiles of <= kTileMaxThreads element threads,
-// prefer shapes whose sides divide the grid (no ragged tiles) and the least
-// recomputed halo; the z depth is left to the launch (kz = 0, launch_kz).
-TileShape heuristic_shape(const VoxGeom& g, int word) {
+// Shape of the damage kernels' bricks (class 2): among owned-node tiles of <= kTileMaxThreads element
+// threads, prefer shapes whose sides divide the grid (no ragged tiles) and the least recomputed halo; the z
+// depth is left to the launch (kz = 0, launch_kz).
+TileShape heuristic_shape(const VoxGeom& g) {
   static const int cand[][2] = {{16, 12}, {12, 16}, {14, 14}, {24, 8}, {16, 8}, {8, 16}, {20, 8}, {32, 4},
                                 {12, 12}, {10, 10}, {8, 8},   {6, 6},   {4, 4},  {2, 2},  {1, 1}};
   TileShape best{1, 1, 1};
@@ -1206,11 +1298,10 @@ TileShape heuristic_shape(const VoxGeom& g, int word) {
     }
   }
   best.kz = 0;
-  (void)word;
   return best;
 }
 
-// Z depth of a tile whose shape leaves it to the launch (kz = 0), from the
+// Z depth of a damage tile whose shape leaves it to the launch (kz = 0), from the
 // number of blocks that can be resident at once (`capacity`): the fewest
 // rounds of resident blocks, each round costing one tile's kz + 1 element
 // layers plus its two-layer prologue.  A power-of-two depth leaves a second,
@@ -1225,6 +1316,71 @@ int launch_kz(long long tiles_xy, int rz, long long capacity) {
     if (cost < best_cost - 1e-9) {
       best_cost = cost;
       best = kz;
+    }
+  }
+  return best;
+}
+
+// Modelled time of an elastic march: `tiles` bricks of kz node layers and `warps` warps, per_sm of them resident
+// on each of `sms` SMs.  A round of resident bricks runs kz + 1 element layers plus a prologue of about one;
+// a layer costs a fixed latency (two barriers and the element's dependent chain) and issue time in proportion
+// to the warps that share a scheduler.  The coefficients (microseconds) are fitted to sweeps of shape and depth;
+// the model then gives, on 64^3, 24.6 us for FP32 16 x 8 x 5 (measured 24.6), 26.6 for 16 x 8 x 6 (26.7), 29.9
+// for 16 x 8 x 4 (28.9), and in FP64 33.1 for 16 x 14 x 10 (32.9), 42.8 for 16 x 8 x 16 (43.1).
+double march_cost(int word, int warps, long long tiles, int per_sm, int sms, int kz) {
+  const double a = word == 4 ? 0.82 : 1.5, b = word == 4 ? 0.5 : 0.42;
+  const long long cap = std::min<long long>((long long)per_sm * sms, kMaxPartials);
+  const long long full = tiles / cap, rem = tiles % cap;
+  // (the last term prefers fewer warps between equals)
+  auto layer = [&](long long blocks) {
+    return a + b * double((blocks * warps + 3) / 4) + 0.01 * double(blocks * warps);
+  };
+  double c = double(full) * layer((cap + sms - 1) / sms);
+  if (rem) c += layer((rem + sms - 1) / sms);
+  return c * (kz + 2);
+}
+
+// The depth with the least modelled time; its cost through *cost.  Only depths that lower the number of
+// z slabs differ in their bricks, so one depth per slab count is looked at.
+int mech_kz(int word, int threads, long long tiles_xy, int rz, int per_sm, int sms, double* cost = nullptr) {
+  int best = 1;
+  double best_cost = 1e300;
+  for (int slabs = 1; slabs <= rz; ++slabs) {
+    const int kz = (rz + slabs - 1) / slabs;
+    const int used = (rz + kz - 1) / kz;
+    if (used < slabs) continue;  // the same depth as fewer slabs
+    const double c = march_cost(word, threads / 32, tiles_xy * used, per_sm, sms, kz);
+    if (c < best_cost - 1e-9) {
+      best_cost = c;
+      best = kz;
+    }
+  }
+  if (cost) *cost = best_cost;
+  return best;
+}
+
+// Shape of the elastic action's bricks (classes 0 and 1): the least modelled time.  In FP64 one block of up to
+// 256 threads fits an SM, so a shape that fills its eight warps wins (192^3: 16 x 14 508 us, 16 x 8 with five
+// warps 805 us); in FP32 about sixteen warps fit either way (285 against 302 us) and the ragged rest of the
+// grid decides.  Shapes without a kernel of their own run the one with run-time offsets, about a tenth slower.
+TileShape mech_shape(const VoxGeom& g, int word) {
+  static const int cand[][2] = {{16, 14}, {16, 8}, {14, 7}, {8, 8}, {16, 12}, {15, 15}, {14, 14}, {12, 12}, {10, 10}};
+  constexpr int kSms = 148;
+  TileShape best{1, 1, 0};
+  double best_cost = 1e300;
+  for (const auto& c : cand) {
+    const TileShape t{std::min(c[0], g.rx), std::min(c[1], g.ry), 0};
+    if (!tile_ok(t)) continue;
+    const int threads = tile_threads(t);
+    const int per_sm = word == 4 ? 512 / threads : (threads > 128 ? 1 : 256 / threads);
+    const long long tiles = (long long)((g.rx + t.ox - 1) / t.ox) * ((g.ry + t.oy - 1) / t.oy);
+    double cost;
+    mech_kz(word, threads, tiles, g.rz, per_sm, kSms, &cost);
+    const bool own = (t.ox == 16 && (t.oy == 14 || t.oy == 8)) || (t.ox == 14 && t.oy == 7) || (t.ox == 8 && t.oy == 8);
+    if (!own) cost *= 1.1;
+    if (cost < best_cost - 1e-9) {
+      best_cost = cost;
+      best = t;
     }
   }
   return best;
@@ -1332,7 +1488,7 @@ int launch_variant_t(const TileArgs<T>& a, const VoxMat<T>& m, cudaStream_t s, c
   const long long tiles_xy = (long long)((v.rx + a.ts.ox - 1) / a.ts.ox) * ((v.ry + a.ts.oy - 1) / a.ts.oy);
   const long long cap = std::min<long long>((long long)per_sm * sms, kMaxPartials);
   TileArgs<T> b = a;
-  if (b.ts.kz <= 0) b.ts.kz = launch_kz(tiles_xy, v.rz, cap);
+  if (b.ts.kz <= 0) b.ts.kz = mech_kz((int)sizeof(T), threads, tiles_xy, v.rz, per_sm, sms);
   const long long n_tiles = tiles_xy * ((v.rz + b.ts.kz - 1) / b.ts.kz);
   const long long grid = std::min<long long>(n_tiles, cap);
   { note_launch(); kern<<<(int)grid, threads, smem, s>>>(b, m, mx, md); }
@@ -1343,8 +1499,11 @@ template <typename T, int COEF, int MODE, int OX, int OY>
 int launch_variant(const TileArgs<T>& a, const VoxMat<T>& m, cudaStream_t s) {
   CUtensorMap mx, md;
   const bool tma = tile_tensor_maps<T>(a, &mx, &md);
-  return tma ? launch_variant_t<T, COEF, MODE, OX, OY, true>(a, m, s, mx, md)
-             : launch_variant_t<T, COEF, MODE, OX, OY, false>(a, m, s, mx, md);
+  if (tma) {  // opt-in: compiled for 16 x 8 bricks and for any shape
+    constexpr bool own = OX == 16 && OY == 8;
+    return launch_variant_t<T, COEF, MODE, own ? OX : 0, own ? OY : 0, true>(a, m, s, mx, md);
+  }
+  return launch_variant_t<T, COEF, MODE, OX, OY, false>(a, m, s, mx, md);
 }
 
 }  // namespace
@@ -1360,7 +1519,17 @@ bool tile_shape_lookup(const VoxGeom& g, int word, int cls, TileShape* t) {
 TileShape tile_shape_for(const VoxGeom& g, int word, int cls) {
   TileShape t;
   if (tile_shape_lookup(g, word, cls, &t)) return t;
-  return heuristic_shape(g, word);
+  if (cls == 2) return heuristic_shape(g);
+  // the model's choice, remembered per host thread: it depends on the grid alone
+  using Key = decltype(shape_key(g, word, cls));
+  static thread_local std::vector<std::pair<Key, TileShape>> seen;
+  const Key key = shape_key(g, word, 0);
+  for (const auto& s : seen)
+    if (s.first == key) return s.second;
+  if (seen.size() >= 64) seen.clear();
+  t = mech_shape(g, word);
+  seen.emplace_back(key, t);
+  return t;
 }
 
 void tile_shape_record(const VoxGeom& g, int word, int cls, const TileShape& t) {
@@ -1390,109 +1559,21 @@ TileShape clamp_shape(TileShape t, const VoxGeom& v) {
   return t;
 }
 
-// The packed FP32 kernel (two elements per thread in float2 lanes) is opt-in
-// (PHASTB_TILE2=1): with twice the live registers per thread it keeps 9 warps
-// per SM resident instead of 15, and measured 38.8 us against the scalar
-// kernel's 31.8 us per 64^3 action (0.442 against 0.451 ms at 192^3), so the
-// scalar kernel stays the default.
-bool tile2_enabled() {
-  static const bool on = [] {
-    const char* e = std::getenv("PHASTB_TILE2");
-    return e && e[0] == '1';
-  }();
-  return on;
-}
-
-template <int COEF, int MODE, int OX, int OY>
-int launch_variant2(const TileArgs<float>& a, const VoxMat<float>& m, cudaStream_t s) {
-  auto kern = h8_tile2_kernel<COEF, MODE, OX, OY>;
-  size_t off_qp = 0, off_cheb = 0;
-  const size_t smem = tile_layout<float>(a.ts.ox, a.ts.oy, COEF == kCoefQP, MODE == kModeCheb, &off_qp, &off_cheb);
-  const int threads = tile2_threads(a.ts);
-  static std::mutex mu;
-  static size_t smem_set = 0;
-  static std::map<std::pair<int, size_t>, int> occ;
-  int per_sm = 1;
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    if (smem > smem_set) {
-      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-        cudaGetLastError();
-        return PHASTB_ERR_CUDA;
-      }
-      smem_set = smem;
-    }
-    auto it = occ.find({threads, smem});
-    if (it == occ.end()) {
-      int b = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kern, threads, smem) != cudaSuccess) {
-        cudaGetLastError();
-        b = 1;
-      }
-      it = occ.emplace(std::make_pair(threads, smem), b < 1 ? 1 : b).first;
-    }
-    per_sm = it->second;
-  }
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const VoxGeom& v = a.g;
-  const long long tiles_xy = (long long)((v.rx + a.ts.ox - 1) / a.ts.ox) * ((v.ry + a.ts.oy - 1) / a.ts.oy);
-  const long long cap = std::min<long long>((long long)per_sm * sms, kMaxPartials);
-  TileArgs<float> b = a;
-  if (b.ts.kz <= 0) b.ts.kz = launch_kz(tiles_xy, v.rz, cap);
-  const long long n_tiles = tiles_xy * ((v.rz + b.ts.kz - 1) / b.ts.kz);
-  const long long grid = std::min<long long>(n_tiles, cap);
-  { note_launch(); kern<<<(int)grid, threads, smem, s>>>(b, m); }
-  return last_launch_status();
-}
-
-template <int COEF, int MODE>
-int by_shape2(const TileArgs<float>& a, const VoxMat<float>& m, cudaStream_t s) {
-  const int ox = a.ts.ox, oy = a.ts.oy;
-  if (ox == 16 && oy == 8) return launch_variant2<COEF, MODE, 16, 8>(a, m, s);
-  if (ox == 16 && oy == 12) return launch_variant2<COEF, MODE, 16, 12>(a, m, s);
-  if (ox == 8 && oy == 8) return launch_variant2<COEF, MODE, 8, 8>(a, m, s);
-  return launch_variant2<COEF, MODE, 0, 0>(a, m, s);
-}
-
-// Packed-kernel dispatch for FP32; PHASTB_UNSUPPORTED when it does not apply.
-template <typename T>
-int dispatch2(const TileArgs<T>& a, const VoxMat<T>& m, int coef, int mode, cudaStream_t s) {
-  if constexpr (!std::is_same<T, float>::value) {
-    return PHASTB_UNSUPPORTED;
-  } else {
-    if (!tile2_enabled() || !tile2_ok(a.ts)) return PHASTB_UNSUPPORTED;
-    switch (coef * 8 + mode) {
-      case kCoefIso * 8 + kModeApply: return by_shape2<kCoefIso, kModeApply>(a, m, s);
-      case kCoefIso * 8 + kModeDot: return by_shape2<kCoefIso, kModeDot>(a, m, s);
-      case kCoefIso * 8 + kModeEnergy: return launch_variant2<kCoefIso, kModeEnergy, 0, 0>(a, m, s);
-      case kCoefIso * 8 + kModeCheb: return by_shape2<kCoefIso, kModeCheb>(a, m, s);
-      case kCoefIso * 8 + kModeNodal: return by_shape2<kCoefIso, kModeNodal>(a, m, s);
-      case kCoefQP * 8 + kModeApply: return by_shape2<kCoefQP, kModeApply>(a, m, s);
-      case kCoefQP * 8 + kModeCheb: return by_shape2<kCoefQP, kModeCheb>(a, m, s);
-      default: return PHASTB_UNSUPPORTED;
-    }
-  }
-}
-
 // The hot variants are also compiled for a few fixed tile shapes (every
 // shared-memory offset then becomes a constant); other shapes run the generic
 // kernel.
 template <typename T, int COEF, int MODE>
 int by_shape(const TileArgs<T>& a, const VoxMat<T>& m, cudaStream_t s) {
   const int ox = a.ts.ox, oy = a.ts.oy;
+  if (ox == 16 && oy == 14) return launch_variant<T, COEF, MODE, 16, 14>(a, m, s);
   if (ox == 16 && oy == 8) return launch_variant<T, COEF, MODE, 16, 8>(a, m, s);
-  if (ox == 32 && oy == 4) return launch_variant<T, COEF, MODE, 32, 4>(a, m, s);
+  if (ox == 14 && oy == 7) return launch_variant<T, COEF, MODE, 14, 7>(a, m, s);
   if (ox == 8 && oy == 8) return launch_variant<T, COEF, MODE, 8, 8>(a, m, s);
-  if (ox == 8 && oy == 4) return launch_variant<T, COEF, MODE, 8, 4>(a, m, s);
-  if (ox == 4 && oy == 4) return launch_variant<T, COEF, MODE, 4, 4>(a, m, s);
   return launch_variant<T, COEF, MODE, 0, 0>(a, m, s);
 }
 
 template <typename T>
 int dispatch(const TileArgs<T>& a, const VoxMat<T>& m, int coef, int mode, cudaStream_t s) {
-  const int st2 = dispatch2<T>(a, m, coef, mode, s);
-  if (st2 != PHASTB_UNSUPPORTED) return st2;
   switch (coef * 8 + mode) {
     case kCoefIso * 8 + kModeApply: return by_shape<T, kCoefIso, kModeApply>(a, m, s);
     case kCoefIso * 8 + kModeDot: return by_shape<T, kCoefIso, kModeDot>(a, m, s);
@@ -1526,7 +1607,7 @@ int tune_shape(TileArgs<T> a, const VoxMat<T>& m, int coef, int mode, cudaStream
   }
   int st = PHASTB_OK;
   float best = 1e30f;
-  TileShape bs = clamp_shape(heuristic_shape(a.g, (int)sizeof(T)), a.g);
+  TileShape bs = clamp_shape(mech_shape(a.g, (int)sizeof(T)), a.g);
   std::vector<TileShape> seen;
   for (const auto& c : cand) {
     for (int kz : kzs) {
@@ -1577,6 +1658,7 @@ TileArgs<T> tile_args(const VoxGeom& v, int cls) {
   a.k.y2 = T(kC2 / v.hy);
   a.k.z1 = T(kC1 / v.hz);
   a.k.z2 = T(kC2 / v.hz);
+  set_modal_k(a.k, v);
   return a;
 }
 
@@ -1873,7 +1955,7 @@ __device__ __forceinline__ TileK<T> batch_k(const BatchCell& c) {
 // One brick of one cell per block: the block builds its cell's arguments in shared
 // memory and runs the single-grid tile body with its brick index inside the cell.
 template <typename T, int MODE, int OX, int OY, int COEF = kCoefIso>
-__global__ void __launch_bounds__(kTileMaxThreads, sizeof(T) == 4 ? 2 : 1)
+__global__ void __launch_bounds__(TileBounds<T, OX, OY>::threads, TileBounds<T, OX, OY>::blocks)
     h8_tile_batch_kernel(TileBatchArgs<T> b, VoxMat<T> m) {
   __shared__ TileArgs<T> sa;
   const int2 wk = b.work[blockIdx.x];

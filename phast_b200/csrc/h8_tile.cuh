@@ -1,14 +1,15 @@
 // Tiled, z-marching voxel H8 elastic action (one kernel, no element scratch).
 //
 // A block owns an ox x oy x kz brick of reduced nodes and marches through its
-// node layers in z.  For each element layer it stages the two bounding node
-// layers (u and d) of the brick plus a one-node halo in shared memory, every
-// thread computes one element of the (ox+1) x (oy+1) element tile (the halo
-// row/column elements are recomputed by the neighbouring bricks), writes the
-// element's lower- and upper-face nodal forces to shared memory, and each
-// owned node then sums its four lower-face contributions of this layer and the
-// four upper-face contributions of the previous layer in a fixed order: the
-// result is deterministic and independent of the tile shape's schedule.
+// node layers in z.  For each element layer it stages the upper node layer (u and
+// d) of the brick plus a one-node halo in shared memory, and every thread computes
+// one element of the (ox+1) x (oy+1) element tile (the halo row/column elements
+// are recomputed by the neighbouring bricks).  A thread stays on its element column,
+// so what it formed from a node layer as the upper face of one element it keeps in
+// registers as the lower face of the next, and the forces of the two elements that
+// share a face are added there too; one set of corner forces per node layer goes
+// through shared memory, where each owned node sums its four corners in a fixed
+// order: the result is deterministic and independent of the tile shape's schedule.
 //
 // The degradation g(d) at the Gauss points and the macro-strain E rows
 // (Pt sum_q w g sigma) are fused; optionally the kernel also returns x . y
@@ -46,15 +47,17 @@ __host__ __device__ inline size_t tile_stage_offset(int nt, int exy, int node_wo
 // per-Gauss-point coarse operators, H of the damage action.
 constexpr int kStageQP = 16, kStageH = 8;
 
-// Dynamic shared memory of h8_tile_kernel: node buffers [3][4][nt] and face
-// buffers [2][12][exy]; then, 16-byte aligned, with per-Gauss-point moduli two
-// element layers of staged (lam_q, mu_q), 16 words per element; then, for a
-// Chebyshev step, two layers of the owned nodes' staged (res, invd, xs) [2][9][ox*oy].
+// Dynamic shared memory of h8_tile_kernel: node buffers [3][nt][4] (ux, uy, uz, d
+// of a node side by side) and the corner forces [12][exy] of one node layer
+// and then, 16-byte aligned, with per-Gauss-point moduli two element layers of staged
+// (lam_q, mu_q), 16 words per element; then, for a Chebyshev step, two layers of the
+// owned nodes' staged (res, invd, xs) [2][9][ox*oy].
 // Returns the total bytes; *off_qp and *off_cheb receive the two offsets.
+constexpr int kFaceWords = 12;
 template <typename T>
 __host__ __device__ inline size_t tile_layout(int ox, int oy, bool qp, bool cheb, size_t* off_qp, size_t* off_cheb) {
   const int nt = (ox + 2) * (oy + 2), exy = (ox + 1) * (oy + 1);
-  size_t o = tile_stage_offset<T>(nt, exy, 12, 24);
+  size_t o = tile_stage_offset<T>(nt, exy, 12, kFaceWords);
   *off_qp = o;
   if (qp) o += sizeof(T) * 2 * kStageQP * (size_t)exy;
   *off_cheb = o;
@@ -90,7 +93,7 @@ __host__ __device__ inline size_t tma_dbytes(int ox, int oy) {
 }
 
 // Dynamic shared memory of the TMA variant, relative to the 128-byte aligned
-// base: [3 u~ layer buffers][3 d layer buffers][face buffers [2][12][exy]], then
+// base: [3 u~ layer buffers][3 d layer buffers][corner forces [12][exy]], then
 // the staged per-element arrays and Chebyshev node data as in tile_layout.
 // Returns the bytes to request (128 bytes of slack for the realignment).
 template <typename T>
@@ -99,7 +102,7 @@ __host__ __device__ inline size_t tile_layout_tma(int ox, int oy, bool qp, bool 
   const int exy = (ox + 1) * (oy + 1);
   size_t o = 3 * (tma_xbytes<T>(ox, oy) + tma_dbytes<T>(ox, oy));
   *off_face = o;
-  o += sizeof(T) * 24 * (size_t)exy;
+  o += sizeof(T) * kFaceWords * (size_t)exy;
   o = (o + 15) / 16 * 16;
   *off_qp = o;
   if (qp) o += sizeof(T) * 2 * kStageQP * (size_t)exy;
@@ -125,7 +128,21 @@ template <typename T>
 struct TileK {
   T c1, c2;                  // N1 = [[c1, c2], [c2, c1]]
   T x1, x2, y1, y2, z1, z2;  // c1/h, c2/h per axis
+  // modal form: g = 1/sqrt(3) (the Gauss coordinate), and per axis a = 1/(4 h), b = a g
+  T g, ax, ay, az, bx, by, bz;
 };
+
+template <typename T>
+void set_modal_k(TileK<T>& k, const VoxGeom& v) {
+  const double g = 0.57735026918962576451;
+  k.g = T(g);
+  k.ax = T(0.25 / v.hx);
+  k.ay = T(0.25 / v.hy);
+  k.az = T(0.25 / v.hz);
+  k.bx = T(0.25 * g / v.hx);
+  k.by = T(0.25 * g / v.hy);
+  k.bz = T(0.25 * g / v.hz);
+}
 
 template <typename T>
 struct TileArgs {
