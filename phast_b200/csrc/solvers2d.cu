@@ -1,6 +1,7 @@
 // 2D solver drivers over the structured-Q4 operators: the bound-projected
 // PCG damage solve and the quasi-static Newton / matrix-free CG mechanics.
 #include "engine.cuh"
+#include "q4_krylov.cuh"
 
 #include <cstddef>
 #include <cstring>
@@ -175,7 +176,7 @@ using ForceEval = int (*)(const void* ctx, const double* u, double* f, cudaStrea
 static int qs_newton(int n2, const LinOp<double>& K, ForceEval force, const void* fctx, const double* f_ext,
                      const uint8_t* bc_mask, const double* bc_vals, double* u, double tol, double cg_tol,
                      int cg_max_iter, int max_iter, int line_search, int ls_max_steps, double ls_min_alpha,
-                     double ls_c, int* info, void* workspace, cudaStream_t s) {
+                     double ls_c, int* info, void* workspace, cudaStream_t s, const Q4MechSys* grid = nullptr) {
   char* p = static_cast<char*>(workspace);
   PcgWs<double> w = pcg_ws<double>(p, n2);
   p += pcg_ws_bytes<double>(n2);
@@ -221,8 +222,11 @@ static int qs_newton(int n2, const LinOp<double>& K, ForceEval force, const void
     // du = CG(K(d) restricted to free dofs, res)
     { note_launch(); zero_kernel<<<G, kThreads, 0, s>>>(n2, du); }
     PcgResult pr{};
+    const PcgLoop loop = [&](int maxiter) {
+      return q4_pcg_persistent(*grid, w, ut, du, maxiter, 50, PCG_PERIODIC, s);  // ut, ub: free here
+    };
     if ((st = pcg_run<double>(K, n2, w, res, nullptr, nullptr, du, cg_tol, cg_max_iter, 50, PCG_PERIODIC, 0.0,
-                              &pr, s)))
+                              &pr, s, grid ? &loop : nullptr)))
       return st;
     total_cg += pr.iterations;
     if (pr.breakdown || pr.nonfinite) {
@@ -288,11 +292,20 @@ int phastb_q4_damage_solve(const phastb_q4_grid* g, const double* Hq, double gc_
   if (scope.status()) return scope.status();
   cudaStream_t s = scope.get();
   PpcgWs w = ppcg_ws(workspace, n);
-  int st = phastb_q4_damage_prepare(g, Hq, gc_over_l0, gc_over_l0_e, gcl0, gcl0_e, w.b, w.minv, (void*)s);
+  int inf[2] = {0, 0};
+  int st = q4_ppcg_persistent(Q4DamageSys{*g, Hq, gc_over_l0, gc_over_l0_e, gcl0, gcl0_e, nullptr}, w, d_prev, d_init,
+                              fixed, fixed_vals, tol, max_iter, check_every, d_out, inf, s);
+  if (st != PHASTB_UNSUPPORTED) {
+    if (info) {
+      info[0] = inf[0];
+      info[1] = inf[1];
+    }
+    return st;
+  }
+  st = phastb_q4_damage_prepare(g, Hq, gc_over_l0, gc_over_l0_e, gcl0, gcl0_e, w.b, w.minv, (void*)s);
   if (st) return st;
   Q4DamageCtx ctx{*g, Hq, gc_over_l0, gc_over_l0_e, gcl0, gcl0_e, nullptr};
   LinOp<double> A{q4_damage_op, &ctx, sizeof(ctx)};
-  int inf[2] = {0, 0};
   st = ppcg_solve(A, n, w, d_prev, d_init, fixed, fixed_vals, tol, max_iter, check_every, d_out, inf, s);
   if (info) {
     info[0] = inf[0];
@@ -302,7 +315,8 @@ int phastb_q4_damage_solve(const phastb_q4_grid* g, const double* Hq, double gc_
 }
 
 size_t phastb_q4_damage_linear_workspace_bytes(int n_nodes) {
-  return pcg_ws_bytes<double>(n_nodes) + 2 * align_up(sizeof(double) * (size_t)n_nodes) + red_ws_bytes();
+  // the engine, the right-hand side and inverse diagonal, the reductions, the persistent solve's rim words
+  return pcg_ws_bytes<double>(n_nodes) + 4 * align_up(sizeof(double) * (size_t)n_nodes) + red_ws_bytes();
 }
 
 int phastb_q4_damage_linear_solve(const phastb_q4_grid* g, const double* Hq, double gc_over_l0,
@@ -323,6 +337,7 @@ int phastb_q4_damage_linear_solve(const phastb_q4_grid* g, const double* Hq, dou
   double* bf = reinterpret_cast<double*>(p);
   double* minv = reinterpret_cast<double*>(p + vb);
   RedWs rw = red_ws(p + 2 * vb);
+  void* tagged = p + 2 * vb + red_ws_bytes();
   int st;
   if ((st = red_ws_reset(rw, s))) return st;
   // Jacobi inverse of the full operator (the b output of prepare is not needed)
@@ -334,11 +349,15 @@ int phastb_q4_damage_linear_solve(const phastb_q4_grid* g, const double* Hq, dou
   if (rinfo) rinfo[0] = bn;
   Q4DamageCtx ctx{*g, Hq, gc_over_l0, gc_over_l0_e, gcl0, gcl0_e, fixed};
   LinOp<double> A{q4_damage_op, &ctx, sizeof(ctx)};
+  const PcgLoop loop = [&](int maxiter) {
+    return q4_pcg_persistent(Q4DamageSys{*g, Hq, gc_over_l0, gc_over_l0_e, gcl0, gcl0_e, fixed}, w, minv, tagged,
+                             x_out, maxiter, check_every, PCG_FREEZE, s);
+  };
   PcgResult pr{};
   if (bn == 0.0) {
     pr.converged = 1;
   } else if ((st = pcg_run<double>(A, n, w, bf, minv, nullptr, x_out, rtol * bn, max_iter, check_every, PCG_FREEZE,
-                                   0.0, &pr, s))) {
+                                   0.0, &pr, s, &loop))) {
     return st;
   }
   if (info) {
@@ -399,8 +418,9 @@ int phastb_q4_qs_solve(const phastb_q4_grid* g, const phastb_q4_material* m, con
   tctx.u = u;
   LinOp<double> K = tangent ? LinOp<double>{q4_tangent_op, &tctx, sizeof(tctx)}
                             : LinOp<double>{q4_force_op, &kctx, sizeof(kctx)};
+  const Q4MechSys sys{*g, *m, d, tangent ? u : nullptr, bc_mask};
   return qs_newton(n2, K, q4_force_eval, &kctx, f_ext, bc_mask, bc_vals, u, tol, cg_tol, cg_max_iter, max_iter,
-                   line_search, ls_max_steps, ls_min_alpha, ls_c, info, workspace, scope.get());
+                   line_search, ls_max_steps, ls_min_alpha, ls_c, info, workspace, scope.get(), &sys);
 }
 
 size_t phastb_t3_qs_workspace_bytes(int n_nodes) { return phastb_q4_qs_workspace_bytes(n_nodes); }
