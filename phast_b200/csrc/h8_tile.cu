@@ -1,5 +1,6 @@
 // Tiled z-marching voxel H8 elastic action (see h8_tile.cuh).
 #include "h8_tile.cuh"
+#include "h8_march.cuh"
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include "engine.cuh"
@@ -15,50 +16,6 @@
 namespace phastb {
 
 namespace {
-
-// Index of a node coordinate along one axis after the periodic wrap; -1 when
-// the coordinate lies outside a non-periodic grid.  |c| stays within one
-// period because tiles are never wider than the grid.
-__device__ __forceinline__ int wrap_node(int c, int n, int r, int periodic) {
-  if (periodic) return c < 0 ? c + n : (c >= n ? c - n : c);
-  return (c >= 0 && c < r) ? c : -1;
-}
-
-__device__ __forceinline__ int wrap_elem(int c, int n, int periodic) {
-  if (periodic) return c < 0 ? c + n : (c >= n ? c - n : c);
-  return (c >= 0 && c < n) ? c : -1;
-}
-
-// Asynchronous global -> shared copies (cp.async, 16 bytes, L2 only).  A thread
-// stages the per-element arrays of the NEXT element layer into its own slot of
-// a two-buffer shared array and waits for its own group before reading it, so
-// no barrier is needed for these slots; both addresses must be 16-byte aligned.
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-// One word (4 or 8 bytes, naturally aligned) with cp.async.
-template <typename T>
-__device__ __forceinline__ void cp_async_word(T* smem, const T* gmem) {
-  static_assert(sizeof(T) == 4 || sizeof(T) == 8, "cp.async copies 4, 8 or 16 bytes");
-  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(s), "l"(gmem), "n"(sizeof(T)) : "memory");
-}
-// One word, or zero where `live` is false (the source is then not read).
-template <typename T>
-__device__ __forceinline__ void cp_async_word_or_zero(T* smem, const T* gmem, bool live) {
-  static_assert(sizeof(T) == 4 || sizeof(T) == 8, "cp.async copies 4, 8 or 16 bytes");
-  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-  const unsigned n = live ? (unsigned)sizeof(T) : 0u;
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(s), "l"(gmem), "n"(sizeof(T)), "r"(n)
-               : "memory");
-}
-__device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
@@ -113,41 +70,6 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
 }
 __device__ __forceinline__ int floor_mult(int v, int m) { return (v >= 0 ? v / m : -((-v + m - 1) / m)) * m; }
 
-// Staged per-element arrays live chunk-major in shared memory: chunk c (16
-// bytes) of the element owned by thread t sits at base + (c * n + t) * 16, so a
-// warp reading one chunk touches consecutive 16-byte units (no bank conflicts).
-template <typename T>
-struct Vec16;
-template <>
-struct Vec16<float> {
-  using type = float4;
-};
-template <>
-struct Vec16<double> {
-  using type = double2;
-};
-
-// Copies n_chunks 16-byte chunks of src into chunks c0.. of thread t's column.
-__device__ __forceinline__ void stage_chunks(unsigned char* base, int n, int t, int c0, const void* src,
-                                             int n_chunks) {
-  for (int c = 0; c < n_chunks; ++c)
-    cp_async16(base + ((size_t)(c0 + c) * n + t) * 16, static_cast<const unsigned char*>(src) + 16 * c);
-}
-
-// Reads W words of thread t's staged column (W * sizeof(T) a multiple of 16).
-template <typename T, int W>
-__device__ __forceinline__ void load_chunks(const unsigned char* base, int n, int t, T (&out)[W]) {
-  using V = typename Vec16<T>::type;
-  constexpr int per = 16 / sizeof(T);
-#pragma unroll
-  for (int c = 0; c < W / per; ++c) {
-    const V v = *reinterpret_cast<const V*>(base + ((size_t)c * n + t) * 16);
-    const T* pv = reinterpret_cast<const T*>(&v);
-#pragma unroll
-    for (int j = 0; j < per; ++j) out[c * per + j] = pv[j];
-  }
-}
-
 // A thread's (at most two) nodes of a layer, in registers (the wrapped halo nodes
 // that TMA staging patches).
 template <typename T>
@@ -168,80 +90,6 @@ __device__ __forceinline__ void get4(const double* p, double (&v)[4]) {
   v[1] = q.y;
   v[2] = r.x;
   v[3] = r.y;
-}
-
-template <typename T>
-__device__ __forceinline__ void ip2(T a0, T a1, T c1, T c2, T& q0, T& q1) {
-  q0 = c1 * a0 + c2 * a1;
-  q1 = c2 * a0 + c1 * a1;
-}
-
-// Gradient of a trilinear field u[L] at the Gauss points: Dx[qz][qy],
-// Dy[qz][qx], Dz[qy][qx] (each independent of its own axis).
-template <typename T>
-__device__ __forceinline__ void grad_k(const T* u, const TileK<T>& k, T (&Dx)[2][2], T (&Dy)[2][2],
-                                       T (&Dz)[2][2]) {
-  {
-    T Y[2][2];  // [az][qy]
-#pragma unroll
-    for (int az = 0; az < 2; ++az)
-      ip2(u[1 + 4 * az] - u[4 * az], u[3 + 4 * az] - u[2 + 4 * az], k.c1, k.c2, Y[az][0], Y[az][1]);
-#pragma unroll
-    for (int qy = 0; qy < 2; ++qy) ip2(Y[0][qy], Y[1][qy], k.x1, k.x2, Dx[0][qy], Dx[1][qy]);
-  }
-  {
-    T Y[2][2];  // [az][qx]
-#pragma unroll
-    for (int az = 0; az < 2; ++az)
-      ip2(u[2 + 4 * az] - u[4 * az], u[3 + 4 * az] - u[1 + 4 * az], k.c1, k.c2, Y[az][0], Y[az][1]);
-#pragma unroll
-    for (int qx = 0; qx < 2; ++qx) ip2(Y[0][qx], Y[1][qx], k.y1, k.y2, Dy[0][qx], Dy[1][qx]);
-  }
-  {
-    T Y[2][2];  // [ay][qx]
-#pragma unroll
-    for (int ay = 0; ay < 2; ++ay)
-      ip2(u[4 + 2 * ay] - u[2 * ay], u[5 + 2 * ay] - u[1 + 2 * ay], k.c1, k.c2, Y[ay][0], Y[ay][1]);
-#pragma unroll
-    for (int qx = 0; qx < 2; ++qx) ip2(Y[0][qx], Y[1][qx], k.z1, k.z2, Dz[0][qx], Dz[1][qx]);
-  }
-}
-
-// Transposed gradient: out[L] = sum over the Gauss points of dN_L/dx_a times
-// the summed terms Px[qz][qy], Py[qz][qx], Pz[qy][qx].
-template <typename T>
-__device__ __forceinline__ void grad_k_t(const T (&Px)[2][2], const T (&Py)[2][2], const T (&Pz)[2][2],
-                                         const TileK<T>& k, T* out) {
-  T Ax[2][2], Ay[2][2], Az[2][2];
-  {
-    T Y[2][2];  // [az][qy]
-#pragma unroll
-    for (int qy = 0; qy < 2; ++qy) ip2(Px[0][qy], Px[1][qy], k.x1, k.x2, Y[0][qy], Y[1][qy]);
-#pragma unroll
-    for (int az = 0; az < 2; ++az) ip2(Y[az][0], Y[az][1], k.c1, k.c2, Ax[az][0], Ax[az][1]);  // [az][ay]
-  }
-  {
-    T Y[2][2];  // [az][qx]
-#pragma unroll
-    for (int qx = 0; qx < 2; ++qx) ip2(Py[0][qx], Py[1][qx], k.y1, k.y2, Y[0][qx], Y[1][qx]);
-#pragma unroll
-    for (int az = 0; az < 2; ++az) ip2(Y[az][0], Y[az][1], k.c1, k.c2, Ay[az][0], Ay[az][1]);  // [az][ax]
-  }
-  {
-    T Y[2][2];  // [ay][qx]
-#pragma unroll
-    for (int qx = 0; qx < 2; ++qx) ip2(Pz[0][qx], Pz[1][qx], k.z1, k.z2, Y[0][qx], Y[1][qx]);
-#pragma unroll
-    for (int ay = 0; ay < 2; ++ay) ip2(Y[ay][0], Y[ay][1], k.c1, k.c2, Az[ay][0], Az[ay][1]);  // [ay][ax]
-  }
-#pragma unroll
-  for (int L = 0; L < 8; ++L) {
-    const int ax = L & 1, ay = (L >> 1) & 1, az = L >> 2;
-    const T tx = ax ? Ax[az][ay] : -Ax[az][ay];
-    const T ty = ay ? Ay[az][ax] : -Ay[az][ax];
-    const T tz = az ? Az[ay][ax] : -Az[ay][ax];
-    out[L] = tx + ty + tz;
-  }
 }
 
 // One node layer as an element sees it: the four corner values of u~ in the Haar basis of the
@@ -897,10 +745,11 @@ __global__ void __launch_bounds__(TileBounds<T, OX, OY>::threads, TileBounds<T, 
 
 // Scalar AT2 damage action on the same brick schedule:
 //   y = scale * [Gc_e (M / ell + ell L) d + 2 (1 - kappa) sum_q w H_q N_q N_q^T d]
-// (the element arithmetic of h8_damage_elem_kernel), masked rows zero.  One
-// pass covers every brick of this (persistent) block: node values come from
-// node_val(n), each owned node's result goes to on_owned(n, x_n, y_n), and the
-// return value is this thread's share of sum_n x_n y_n (with DOT).
+// (damage_element), masked rows zero.  One pass covers every brick of this
+// (persistent) block: node values come from node_val(n), each owned node's
+// result goes to on_owned(n, x_n, y_n), and the return value is this thread's
+// share of sum_n x_n y_n (with DOT).  A thread keeps its column's upper face and
+// force in registers, as the elastic march does.
 template <typename T, int OX, int OY, bool DOT, class NodeVal, class OnOwned>
 __device__ __forceinline__ double dtile_pass(const DTileArgs<T>& a, unsigned char* smem_raw, NodeVal node_val,
                                              OnOwned on_owned, const int vb, const int vgrid) {
@@ -909,13 +758,13 @@ __device__ __forceinline__ double dtile_pass(const DTileArgs<T>& a, unsigned cha
   const int ex = ox + 1, exy = ex * (oy + 1);
   const int ntx = ox + 2, nt = ntx * (oy + 2);
   T* nb = reinterpret_cast<T*>(smem_raw);  // [3 buffers][nt]
-  T* FL = nb + 3 * nt;                     // [4 corners][exy]
-  T* FU = FL + 4 * exy;
+  T* FC = nb + 3 * nt;                     // corner results of one node layer, [4 corners][exy]
   // H of this thread's element, staged one element layer ahead, chunk-major [2][chunks][exy]
   constexpr int kHChunks = kStageH * (int)sizeof(T) / 16;
-  unsigned char* HS = smem_raw + tile_stage_offset<T>(nt, exy, 3, 8);
+  unsigned char* HS = smem_raw + tile_stage_offset<T>(nt, exy, 3, 4);
   const int tid = threadIdx.x;
-  const T w = T(g.w), ch = T(2.0 * (1.0 - a.kappa)), sc = T(a.scale);
+  const T wsc = T(g.w * a.scale / 64.0), chw = wsc * T(2.0 * (1.0 - a.kappa));
+  const DElemK<T> ek = damage_elem_k<T>(g, a.scale);
   const int tiles_x = (g.rx + ox - 1) / ox, tiles_y = (g.ry + oy - 1) / oy;
   const int tiles_xy = tiles_x * tiles_y;
   const int n_tiles = tiles_xy * ((g.rz + kz - 1) / kz);
@@ -923,56 +772,68 @@ __device__ __forceinline__ double dtile_pass(const DTileArgs<T>& a, unsigned cha
   const int ni = tid % ox, nj = tid / ox;
   const bool is_elem = tid < exy, is_node = tid < ox * oy;
   const bool h_async = a.H != nullptr && aligned16(a.H);
+  const size_t plane_n = (size_t)g.rx * g.ry, plane_e = (size_t)g.nx * g.ny;
   double accd = 0.0;
-  // issues the copy of element layer ke's H into buffer `buf` (one commit group
-  // per call, empty when there is nothing to copy) and returns its material slot
-  auto stage_elem = [&](int i0, int j0, int ke, int buf) -> int {
-    int sl = 0;
-    if (is_elem) {
-      const int gi = wrap_elem(i0 - 1 + ea, g.nx, g.px);
-      const int gj = wrap_elem(j0 - 1 + eb, g.ny, g.py);
-      const int gk = wrap_elem(ke, g.nz, g.pz);
-      if (gi >= 0 && gj >= 0 && gk >= 0) {
-        const size_t e = (size_t)gi + (size_t)g.nx * ((size_t)gj + (size_t)g.ny * gk);
-        sl = __ldg(a.slot + e);
-        if (h_async) stage_chunks(HS + (size_t)buf * kHChunks * exy * 16, exy, tid, 0, a.H + kStageH * e, kHChunks);
-      }
-    }
-    cp_async_commit();
-    return sl;
-  };
-  auto stage1 = [&](int i0, int j0, int kn, T (&r)[2]) {
-    const int gk = wrap_node(kn, g.nz, g.rz, g.pz);
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int t = tid + h * blockDim.x;
-      T v = T(0);
-      if (t < nt && gk >= 0) {
-        const int gi = wrap_node(i0 - 1 + t % ntx, g.nx, g.rx, g.px);
-        const int gj = wrap_node(j0 - 1 + t / ntx, g.ny, g.ry, g.py);
-        if (gi >= 0 && gj >= 0) v = node_val((size_t)gi + (size_t)g.rx * ((size_t)gj + (size_t)g.ry * gk));
-      }
-      r[h] = v;
-    }
-  };
-  auto store1 = [&](const T (&r)[2], T* buf) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int t = tid + h * blockDim.x;
-      if (t < nt) buf[t] = r[h];
-    }
-  };
   for (int tile = vb; tile < n_tiles; tile += vgrid) {
     const int tz = tile / tiles_xy, txy = tile - tz * tiles_xy;
     const int i0 = (txy % tiles_x) * ox, j0 = (txy / tiles_x) * oy;
     const int k0 = tz * kz, k1 = min(k0 + kz, g.rz);
-    T tdot = T(0), pend = T(0);
+    // in-plane offsets, once per brick (-1: outside the grid or not this thread's)
+    int so[2], eo = -1, no = -1;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int t = tid + h * blockDim.x;
+      so[h] = -1;
+      if (t < nt) {
+        const int gi = wrap_node(i0 - 1 + t % ntx, g.nx, g.rx, g.px);
+        const int gj = wrap_node(j0 - 1 + t / ntx, g.ny, g.ry, g.py);
+        if (gi >= 0 && gj >= 0) so[h] = gi + g.rx * gj;
+      }
+    }
+    if (is_elem) {
+      const int gi = wrap_elem(i0 - 1 + ea, g.nx, g.px);
+      const int gj = wrap_elem(j0 - 1 + eb, g.ny, g.py);
+      if (gi >= 0 && gj >= 0) eo = gi + g.nx * gj;
+    }
+    if (is_node && i0 + ni < g.rx && j0 + nj < g.ry) no = (i0 + ni) + g.rx * (j0 + nj);
+    // issues the copy of element layer ke's H into buffer `buf` (one commit group
+    // per call, empty when there is nothing to copy) and returns its material slot
+    auto stage_elem = [&](int ke, int buf) -> int {
+      const int gk = wrap_elem(ke, g.nz, g.pz);
+      int sl = 0;
+      if (eo >= 0 && gk >= 0) {
+        const size_t e = plane_e * gk + eo;
+        sl = __ldg(a.slot + e);
+        if (h_async) stage_chunks(HS + (size_t)buf * kHChunks * exy * 16, exy, tid, 0, a.H + kStageH * e, kHChunks);
+      }
+      cp_async_commit();
+      return sl;
+    };
+    auto stage1 = [&](int kn, T (&r)[2]) {
+      const int gk = wrap_node(kn, g.nz, g.rz, g.pz);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) r[h] = so[h] >= 0 && gk >= 0 ? node_val(plane_n * gk + so[h]) : T(0);
+    };
+    auto store1 = [&](const T (&r)[2], T* buf) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int t = tid + h * blockDim.x;
+        if (t < nt) buf[t] = r[h];
+      }
+    };
+    auto load_face = [&](const T* buf) {
+      const T* c = buf + eb * ntx + ea;
+      return dface(c[0], c[1], c[ntx], c[ntx + 1]);
+    };
+    T tdot = T(0);
     T pf[2];
-    stage1(i0, j0, k0 - 1, pf);
+    DFace<T> fl;
+    DForce<T> pend{T(0), T(0), T(0), T(0)};
+    stage1(k0 - 1, pf);
     __syncthreads();
     store1(pf, nb);
-    stage1(i0, j0, k0, pf);
-    int sl_next = stage_elem(i0, j0, k0 - 1, 0);
+    stage1(k0, pf);
+    int sl_next = stage_elem(k0 - 1, 0);
     const int K = k1 - k0;
     for (int kk = 0; kk <= K; ++kk) {
       const int ke = k0 - 1 + kk;
@@ -981,79 +842,49 @@ __device__ __forceinline__ double dtile_pass(const DTileArgs<T>& a, unsigned cha
       store1(pf, b1);
       const int sl = sl_next;
       if (kk < K) {
-        stage1(i0, j0, ke + 2, pf);
-        sl_next = stage_elem(i0, j0, ke + 1, (kk + 1) & 1);
+        stage1(ke + 2, pf);
+        sl_next = stage_elem(ke + 1, (kk + 1) & 1);
         cp_async_wait<1>();  // this thread's copy of layer ke has landed
       } else {
         cp_async_wait<0>();
       }
       __syncthreads();
       if (is_elem) {
-        const int gi = wrap_elem(i0 - 1 + ea, g.nx, g.px);
-        const int gj = wrap_elem(j0 - 1 + eb, g.ny, g.py);
+        if (kk == 0) fl = load_face(b0);
+        const DFace<T> fu = load_face(b1);
         const int gk = wrap_elem(ke, g.nz, g.pz);
-        T out[8];
-        if (gi >= 0 && gj >= 0 && gk >= 0) {
-          const size_t e = (size_t)gi + (size_t)g.nx * ((size_t)gj + (size_t)g.ny * gk);
-          const T gc_ell = a.gc_ell[sl], k2 = a.gc_k2[sl];
-          T dd[8], dq[8];
-#pragma unroll
-          for (int L = 0; L < 8; ++L) {
-            const T* bb = (L & 4) ? b1 : b0;
-            dd[L] = bb[(eb + ((L >> 1) & 1)) * ntx + ea + (L & 1)];
-          }
-          interp_sf(dd, dq);
+        DForce<T> lo = pend;
+        pend = DForce<T>{T(0), T(0), T(0), T(0)};
+        if (eo >= 0 && gk >= 0) {
           T hq[kStageH];
           if (h_async) {
             load_chunks<T, kStageH>(HS + (size_t)(kk & 1) * kHChunks * exy * 16, exy, tid, hq);
           } else {
+            const size_t e = plane_e * gk + eo;
 #pragma unroll
             for (int q = 0; q < 8; ++q) hq[q] = a.H ? __ldg(a.H + 8 * e + q) : T(0);
           }
-          T mq[8];
-#pragma unroll
-          for (int q = 0; q < 8; ++q) mq[q] = w * (gc_ell + ch * hq[q]) * dq[q];
-          interp_sf_t(mq, out);
-          T Dx[2][2], Dy[2][2], Dz[2][2];
-          grad_k(dd, a.k, Dx, Dy, Dz);
-#pragma unroll
-          for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-              Dx[i][j] *= k2;
-              Dy[i][j] *= k2;
-              Dz[i][j] *= k2;
-            }
-          T og[8];
-          grad_k_t(Dx, Dy, Dz, a.k, og);
-#pragma unroll
-          for (int L = 0; L < 8; ++L) out[L] = sc * (out[L] + og[L]);
-        } else {
-#pragma unroll
-          for (int L = 0; L < 8; ++L) out[L] = T(0);
+          damage_element(fl, fu, hq, wsc * a.gc_ell[sl], chw, a.gc_k2[sl], ek, lo, pend);
         }
+        fl = fu;
+        if (kk >= 1) {
+          T c[4];
+          dcorners(lo, c);
 #pragma unroll
-        for (int L = 0; L < 4; ++L) {
-          FL[L * exy + tid] = out[L];
-          FU[L * exy + tid] = out[L + 4];
+          for (int L = 0; L < 4; ++L) FC[L * exy + tid] = c[L];
         }
       }
+      if (kk == 0) continue;  // the first element layer only fills pend
       __syncthreads();
-      if (is_node) {
+      if (no >= 0) {
         const int e11 = (ni + 1) + ex * (nj + 1), e01 = ni + ex * (nj + 1);
         const int e10 = (ni + 1) + ex * nj, e00 = ni + ex * nj;
-        const T lo = FL[0 * exy + e11] + FL[1 * exy + e01] + FL[2 * exy + e10] + FL[3 * exy + e00];
-        const T up = FU[0 * exy + e11] + FU[1 * exy + e01] + FU[2 * exy + e10] + FU[3 * exy + e00];
-        const int gi = i0 + ni, gj = j0 + nj;
-        if (kk >= 1 && gi < g.rx && gj < g.ry) {
-          const size_t n = (size_t)gi + (size_t)g.rx * ((size_t)gj + (size_t)g.ry * ke);
-          T v = pend + lo;
-          if (a.mask && __ldg(a.mask + n)) v = T(0);
-          const T xn = b0[(nj + 1) * ntx + ni + 1];
-          on_owned(n, xn, v);
-          if (DOT) tdot += xn * v;
-        }
-        pend = up;
+        const size_t n = plane_n * ke + no;
+        T v = (FC[e11] + FC[exy + e01]) + (FC[2 * exy + e10] + FC[3 * exy + e00]);
+        if (a.mask && __ldg(a.mask + n)) v = T(0);
+        const T xn = b0[(nj + 1) * ntx + ni + 1];
+        on_owned(n, xn, v);
+        if (DOT) tdot += xn * v;
       }
     }
     if (DOT) accd += double(tdot);
@@ -1706,7 +1537,7 @@ template <typename T, int MODE, int OX, int OY>
 int dlaunch_variant(const DTileArgs<T>& a, cudaStream_t s) {
   auto kern = h8_dtile_kernel<T, MODE, OX, OY>;
   const int nt = (a.ts.ox + 2) * (a.ts.oy + 2), exy = (a.ts.ox + 1) * (a.ts.oy + 1);
-  const size_t smem = tile_stage_offset<T>(nt, exy, 3, 8) + sizeof(T) * 2 * kStageH * (size_t)exy;
+  const size_t smem = tile_stage_offset<T>(nt, exy, 3, 4) + sizeof(T) * 2 * kStageH * (size_t)exy;
   const int threads = tile_threads(a.ts);
   static std::mutex mu;
   static size_t smem_set = 0;
@@ -1758,7 +1589,7 @@ template <typename T, int OX, int OY>
 int dpcg_variant(const DTileArgs<T>& a0, const DamagePcgArgs<T>& c0, cudaStream_t s) {
   auto kern = h8_damage_pcg_kernel<T, OX, OY>;
   const int nt = (a0.ts.ox + 2) * (a0.ts.oy + 2), exy = (a0.ts.ox + 1) * (a0.ts.oy + 1);
-  const size_t smem = tile_stage_offset<T>(nt, exy, 3, 8) + sizeof(T) * 2 * kStageH * (size_t)exy;
+  const size_t smem = tile_stage_offset<T>(nt, exy, 3, 4) + sizeof(T) * 2 * kStageH * (size_t)exy;
   const int threads = tile_threads(a0.ts);
   static std::mutex mu;
   static size_t smem_set = 0;
@@ -1899,7 +1730,7 @@ template int h8_damage_tile_launch<float>(const VoxGeom&, const VoxMat<float>&, 
 template <typename T>
 int h8_damage_pcg_launch(const VoxGeom& v, const VoxMat<T>& m, const uint8_t* slot, const T* H, double scale,
                          const uint8_t* mask, const PcgWs<T>& w, T* p_alt, T* x, const T* inv_diag, int maxiter,
-                         int mode, cudaStream_t s) {
+                         int mode, cudaStream_t s, void* tagged) {
   if (mode == PCG_PERIODIC || !persistent_pcg_enabled()) return PHASTB_UNSUPPORTED;
   DTileArgs<T> a;
   std::memset(&a, 0, sizeof(a));
@@ -1915,6 +1746,10 @@ int h8_damage_pcg_launch(const VoxGeom& v, const VoxMat<T>& m, const uint8_t* sl
   a.H = H;
   a.mask = mask;
   if (!tile_ok(a.ts)) return PHASTB_ERR_ARG;
+  if (tagged) {
+    const int st = h8_damage_brick_pcg<T>(a, w, tagged, x, inv_diag, maxiter, mode, s);
+    if (st != PHASTB_UNSUPPORTED) return st;
+  }
   DamagePcgArgs<T> c;
   std::memset(&c, 0, sizeof(c));
   c.n = v.n_red;
@@ -1938,10 +1773,10 @@ int h8_damage_pcg_launch(const VoxGeom& v, const VoxMat<T>& m, const uint8_t* sl
 
 template int h8_damage_pcg_launch<double>(const VoxGeom&, const VoxMat<double>&, const uint8_t*, const double*,
                                           double, const uint8_t*, const PcgWs<double>&, double*, double*,
-                                          const double*, int, int, cudaStream_t);
+                                          const double*, int, int, cudaStream_t, void*);
 template int h8_damage_pcg_launch<float>(const VoxGeom&, const VoxMat<float>&, const uint8_t*, const float*,
                                          double, const uint8_t*, const PcgWs<float>&, float*, float*, const float*,
-                                         int, int, cudaStream_t);
+                                         int, int, cudaStream_t, void*);
 // ------------------------------------------------------------ packed cell batches
 
 template <typename T>
@@ -2067,7 +1902,7 @@ template <typename T, int MODE, int OX, int OY>
 int dtile_batch_variant(const TileBatchArgs<T>& b, const VoxMat<T>& m, cudaStream_t s) {
   auto kern = h8_dtile_batch_kernel<T, MODE, OX, OY>;
   const int nt = (OX + 2) * (OY + 2), exy = (OX + 1) * (OY + 1);
-  const size_t smem = tile_stage_offset<T>(nt, exy, 3, 8) + sizeof(T) * 2 * kStageH * (size_t)exy;
+  const size_t smem = tile_stage_offset<T>(nt, exy, 3, 4) + sizeof(T) * 2 * kStageH * (size_t)exy;
   int st = batch_smem_attr(kern, smem);
   if (st) return st;
   const int threads = ((OX + 1) * (OY + 1) + 31) / 32 * 32;

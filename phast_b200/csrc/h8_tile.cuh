@@ -211,11 +211,17 @@ struct PcgWs;
 // state that pcg_start_kernel left in w (engine.cuh's PcgLoop contract); p_alt
 // is a second direction buffer of n_red values.  PHASTB_UNSUPPORTED when the
 // device cannot run it (or PHASTB_PERSISTENT_PCG=0): the caller iterates with
-// separate launches instead.
+// separate launches instead.  `tagged`: 16 bytes of scratch per node, 16-byte
+// aligned (null: the form that needs none).
 template <typename T>
 int h8_damage_pcg_launch(const VoxGeom& v, const VoxMat<T>& m, const uint8_t* slot, const T* H, double scale,
                          const uint8_t* mask, const PcgWs<T>& w, T* p_alt, T* x, const T* inv_diag, int maxiter,
-                         int mode, cudaStream_t s);
+                         int mode, cudaStream_t s, void* tagged);
+
+// The same with the whole state on the SMs (h8_dpcg.cu); PHASTB_UNSUPPORTED when the cell does not fit.
+template <typename T>
+int h8_damage_brick_pcg(const DTileArgs<T>& d, const PcgWs<T>& w, void* tagged, T* x, const T* inv_diag, int maxiter,
+                        int mode, cudaStream_t s);
 
 // y = A(d) x with fused g(d); optional x . y (DOT) and energy (ENERGY).  ws.out
 // receives the E-row sums (kOutE..), the energy and the dot.

@@ -543,7 +543,9 @@ int box_kkt_run(const VoxGeom& v, const VoxMat<double>& mm, const uint8_t* slot,
     if (!mixed) {
       // all iterations in one persistent launch where the device allows it
       const PcgLoop loop = [&](int mi) {
-        return h8_damage_pcg_launch<double>(v, mm, slot, Hw, scale, fixed, w, p_alt, xd, invd, mi, PCG_STRICT, s);
+        // the element scratch (192 bytes per voxel, at most 8 nodes each) is free during the CG
+        return h8_damage_pcg_launch<double>(v, mm, slot, Hw, scale, fixed, w, p_alt, xd, invd, mi, PCG_STRICT, s,
+                                            scratch);
       };
       if ((st = pcg_run<double>(A, n, w, bf, invd, nullptr, xd, -lin_tol, max_lin, 10, PCG_STRICT, 0.0, &pr, s,
                                 &loop)))
@@ -562,7 +564,7 @@ int box_kkt_run(const VoxGeom& v, const VoxMat<double>& mm, const uint8_t* slot,
       LinOp<float> A32{damage_op32, &c32, sizeof(c32), damage_op_dot32, dw32.out + kOutDot};
       const PcgLoop loop32 = [&](int mi) {
         return h8_damage_pcg_launch<float>(v, m32, slot, H32, scale, fixed, w32, palt32, dx32, invd32, mi,
-                                           PCG_STRICT, s);
+                                           PCG_STRICT, s, scratch);
       };
       int inner = 0, conv = 0;
       for (int k = 0; k < 30 && inner < max_lin; ++k) {
