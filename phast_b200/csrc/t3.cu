@@ -16,6 +16,12 @@
 
 namespace phastb {
 
+// t3_krylov.cu
+size_t t3_ppcg_extra_bytes(int n);
+int t3_ppcg_persistent(const phastb_t3_mesh& mesh, const phastb_t3_damage_model& md, const double* H, const PpcgWs& w,
+                       int* adj, const double* d_prev, const double* d_init, const uint8_t* fixed, const double* vals,
+                       double tol, int max_iter, int check_every, double* d, int* info, cudaStream_t s);
+
 namespace {
 
 struct T3Dev {
@@ -544,7 +550,9 @@ int phastb_t3_damage_prepare(const phastb_t3_mesh* mesh, const double* H, double
   return last_launch_status();
 }
 
-size_t phastb_t3_damage_solve_workspace_bytes(int n_nodes) { return ppcg_ws_bytes(n_nodes); }
+size_t phastb_t3_damage_solve_workspace_bytes(int n_nodes) {
+  return ppcg_ws_bytes(n_nodes) + t3_ppcg_extra_bytes(n_nodes);
+}
 
 int phastb_t3_damage_solve(const phastb_t3_mesh* mesh, const double* H, double gc_over_l0,
                            const double* gc_over_l0_e, double gcl0, const double* gcl0_e, const double* d_prev,
@@ -554,12 +562,28 @@ int phastb_t3_damage_solve(const phastb_t3_mesh* mesh, const double* H, double g
   if (!t3_valid_mesh(mesh) || !d_prev || !d_out || max_iter < 0 || check_every < 1) return PHASTB_ERR_ARG;
   if (fixed && !fixed_vals) return PHASTB_ERR_ARG;
   const int n = mesh->n_nodes;
-  if (!workspace || workspace_bytes < ppcg_ws_bytes(n)) return PHASTB_ERR_WORKSPACE;
+  if (!workspace || workspace_bytes < phastb_t3_damage_solve_workspace_bytes(n)) return PHASTB_ERR_WORKSPACE;
   ScopedStream scope((cudaStream_t)stream);
   if (scope.status()) return scope.status();
   cudaStream_t s = scope.get();
   PpcgWs w = ppcg_ws(workspace, n);
-  int st = phastb_t3_damage_prepare(mesh, H, gc_over_l0, gc_over_l0_e, gcl0, gcl0_e, w.b, w.minv, (void*)s);
+  phastb_t3_damage_model md;
+  std::memset(&md, 0, sizeof(md));
+  md.gcl0 = gcl0;
+  md.gc_over_l0 = gc_over_l0;
+  md.gcl0_e = gcl0_e;
+  md.gc_over_l0_e = gc_over_l0_e;
+  int inf[2] = {0, 0};
+  int st = t3_ppcg_persistent(*mesh, md, H, w, reinterpret_cast<int*>(static_cast<char*>(workspace) + ppcg_ws_bytes(n)),
+                              d_prev, d_init, fixed, fixed_vals, tol, max_iter, check_every, d_out, inf, s);
+  if (st != PHASTB_UNSUPPORTED) {
+    if (info) {
+      info[0] = inf[0];
+      info[1] = inf[1];
+    }
+    return st;
+  }
+  st = phastb_t3_damage_prepare(mesh, H, gc_over_l0, gc_over_l0_e, gcl0, gcl0_e, w.b, w.minv, (void*)s);
   if (st) return st;
   T3DamageCtx ctx;
   std::memset(&ctx, 0, sizeof(ctx));
@@ -570,7 +594,6 @@ int phastb_t3_damage_solve(const phastb_t3_mesh* mesh, const double* H, double g
   ctx.gcl0 = gcl0;
   ctx.gcl0_e = gcl0_e;
   LinOp<double> A{t3_damage_op, &ctx, sizeof(ctx)};
-  int inf[2] = {0, 0};
   st = ppcg_solve(A, n, w, d_prev, d_init, fixed, fixed_vals, tol, max_iter, check_every, d_out, inf, s);
   if (info) {
     info[0] = inf[0];
@@ -615,12 +638,23 @@ int phastb_t3_damage_solve_ex(const phastb_t3_mesh* mesh, const phastb_t3_damage
     return PHASTB_ERR_ARG;
   if (fixed && !fixed_vals) return PHASTB_ERR_ARG;
   const int n = mesh->n_nodes;
-  if (!workspace || workspace_bytes < ppcg_ws_bytes(n)) return PHASTB_ERR_WORKSPACE;
+  if (!workspace || workspace_bytes < phastb_t3_damage_solve_workspace_bytes(n)) return PHASTB_ERR_WORKSPACE;
   ScopedStream scope((cudaStream_t)stream);
   if (scope.status()) return scope.status();
   cudaStream_t s = scope.get();
   PpcgWs w = ppcg_ws(workspace, n);
-  int st = phastb_t3_damage_prepare_ex(mesh, model, H, w.b, w.minv, (void*)s);
+  int inf[2] = {0, 0};
+  int st = t3_ppcg_persistent(*mesh, *model, H, w,
+                              reinterpret_cast<int*>(static_cast<char*>(workspace) + ppcg_ws_bytes(n)), d_prev, d_init,
+                              fixed, fixed_vals, tol, max_iter, check_every, d_out, inf, s);
+  if (st != PHASTB_UNSUPPORTED) {
+    if (info) {
+      info[0] = inf[0];
+      info[1] = inf[1];
+    }
+    return st;
+  }
+  st = phastb_t3_damage_prepare_ex(mesh, model, H, w.b, w.minv, (void*)s);
   if (st) return st;
   T3ModelCtx ctx;
   std::memset(&ctx, 0, sizeof(ctx));
@@ -628,7 +662,6 @@ int phastb_t3_damage_solve_ex(const phastb_t3_mesh* mesh, const phastb_t3_damage
   ctx.model = *model;
   ctx.H = H;
   LinOp<double> A{t3_model_op, &ctx, sizeof(ctx)};
-  int inf[2] = {0, 0};
   st = ppcg_solve(A, n, w, d_prev, d_init, fixed, fixed_vals, tol, max_iter, check_every, d_out, inf, s);
   if (info) {
     info[0] = inf[0];
