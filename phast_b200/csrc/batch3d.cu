@@ -97,10 +97,14 @@ void make_chunks(const std::vector<long long>& off, const std::vector<long long>
                  std::vector<int>* counts) {
   out->clear();
   counts->clear();
+  // up to eight entries per thread, fewer where the batch would leave SMs idle (about eight blocks per SM)
+  long long total = 0;
+  for (long long n : len) total += n;
+  const long long want = std::max<long long>(1, std::min<long long>(8, total / ((long long)kThreads * kMaxBlocks)));
   for (size_t c = 0; c < off.size(); ++c) {
     const long long n = len[c];
     const long long per = (n + (long long)kThreads * kBatchMaxChunks - 1) / ((long long)kThreads * kBatchMaxChunks);
-    const long long ch = (long long)kThreads * std::max<long long>(8, per);
+    const long long ch = (long long)kThreads * std::max(want, per);
     int j = 0;
     for (long long b = 0; b < n; b += ch, ++j)
       out->push_back(BChunk{(int)c, (int)(off[c] + b), (int)(off[c] + std::min(n, b + ch)), j});
@@ -789,9 +793,11 @@ __global__ void bg_first_b_kernel(BVec V, const BatchCell* cells, float* __restr
       bi -= m[(i - cl.mech_off) % 3];
       b[i] = bi;
     }
-    res[i] = bi;
     const float di = invd[i] * bi * it;
-    d[i] = di;
+    if (res) {  // (a smoother of one step needs neither)
+      res[i] = bi;
+      d[i] = di;
+    }
     x[i] = di;
   }
 }
@@ -838,33 +844,38 @@ __global__ void __launch_bounds__(kThreads) bg_restrict_kernel(BVec Vc, const Ba
   const VoxGeom& cg = ccells[c].g;
   const long long fo = fcells[c].mech_off, co = ccells[c].mech_off, no = ccells[c].node_off;
   double v[3] = {0.0, 0.0, 0.0};
-  for (int n = ck.begin + threadIdx.x; n < ck.end; n += blockDim.x) {
-    const int ln = (int)(n - no);
+  // one component of a coarse node per thread (gmg_restrict)
+  for (int t = threadIdx.x; t < 3 * (ck.end - ck.begin); t += blockDim.x) {
+    const int q = t / 3, comp = t - 3 * q, ln = (int)(ck.begin + q - no);
     const int I = ln % cg.rx, rem = ln / cg.rx, J = rem % cg.ry, K = rem / cg.ry;
-    float a0 = 0.f, a1 = 0.f, a2 = 0.f;
-    for (int oz = -1; oz <= 1; ++oz) {
-      const int k = bg_wrap(2 * K + oz, f.nz);
-      const float wz = oz == 0 ? 1.f : 0.5f;
-      for (int oy = -1; oy <= 1; ++oy) {
-        const int j = bg_wrap(2 * J + oy, f.ny);
-        const float wy = oy == 0 ? 1.f : 0.5f;
-        for (int ox = -1; ox <= 1; ++ox) {
-          const int i = bg_wrap(2 * I + ox, f.nx);
-          const float wgt = (ox == 0 ? 1.f : 0.5f) * wy * wz;
-          const long long fn = fo + 3LL * ((long long)i + (long long)f.rx * ((long long)j + (long long)f.ry * k));
-          a0 += wgt * ((mask && mask[fn + 0]) ? 0.f : rf[fn + 0]);
-          a1 += wgt * ((mask && mask[fn + 1]) ? 0.f : rf[fn + 1]);
-          a2 += wgt * ((mask && mask[fn + 2]) ? 0.f : rf[fn + 2]);
-        }
-      }
+    int i[3], j[3], k[3];
+#pragma unroll
+    for (int o = 0; o < 3; ++o) {
+      i[o] = bg_wrap(2 * I + o - 1, f.nx);
+      j[o] = bg_wrap(2 * J + o - 1, f.ny);
+      k[o] = bg_wrap(2 * K + o - 1, f.nz);
     }
-    const long long cn = co + 3LL * ln;
-    rc[cn + 0] = a0;
-    rc[cn + 1] = a1;
-    rc[cn + 2] = a2;
-    v[0] += double(a0);
-    v[1] += double(a1);
-    v[2] += double(a2);
+    float az = 0.f;
+#pragma unroll
+    for (int oz = 0; oz < 3; ++oz) {
+      float ay = 0.f;
+#pragma unroll
+      for (int oy = 0; oy < 3; ++oy) {
+        float r[3];
+#pragma unroll
+        for (int ox = 0; ox < 3; ++ox) {
+          const long long fn =
+              fo + 3LL * ((long long)i[ox] + (long long)f.rx * ((long long)j[oy] + (long long)f.ry * k[oz])) + comp;
+          r[ox] = mask && mask[fn] ? 0.f : __ldg(rf + fn);
+        }
+        ay += (oy == 1 ? 1.f : 0.5f) * (r[1] + 0.5f * (r[0] + r[2]));
+      }
+      az += (oz == 1 ? 1.f : 0.5f) * ay;
+    }
+    rc[co + 3LL * ln + comp] = az;
+    v[0] += comp == 0 ? double(az) : 0.0;
+    v[1] += comp == 1 ? double(az) : 0.0;
+    v[2] += comp == 2 ? double(az) : 0.0;
   }
   seg_fold<3>(v, sum_red, ck, Vc.nchunk[c], [&](const double* f3, RedWs& w) {
     for (int k = 0; k < 3; ++k) w.out[k] = f3[k];
@@ -1300,9 +1311,10 @@ int bg_level_apply(const BGmg& M, int l, const float* x, float* y, cudaStream_t 
 
 // one fused Chebyshev step: res -= A din; dout = c1 din + c2 s_c invd res; x += dout
 int bg_level_cheb(const BGmg& M, int l, const float* din, float* dout, double c1, double c2, bool scaled,
-                  cudaStream_t s) {
+                  cudaStream_t s, bool sum_x = false) {
   const BLevel& L = M.L[l];
   TileBatchArgs<float> a = bg_args(M, l, din);
+  a.ws = sum_x ? L.red : nullptr;
   a.res = L.res;
   a.invd = L.invd;
   a.xs = L.x;
@@ -1316,16 +1328,35 @@ int bg_level_cheb(const BGmg& M, int l, const float* din, float* dout, double c1
 BVec level_mech_vec(const phastb_batch* P) { return mech_vec(P); }
 BVec level_node_vec(const phastb_batch* P) { return node_vec(P); }
 
+// out = b - A x, or with smooth out = x + invd (b - A x) / theta_c (gmg.cu's level_residual; a coarse level's
+// component sums per cell in L.red, the fine level's b . out there)
+int bg_level_residual(const BGmg& M, int l, const float* x, float* out, bool smooth, cudaStream_t s) {
+  const BLevel& L = M.L[l];
+  TileBatchArgs<float> a = bg_args(M, l, x);
+  a.res = L.b;
+  a.invd = L.invd;
+  a.y = out;
+  a.ws = smooth ? L.red : nullptr;
+  a.c2 = 1.0;
+  a.c2_scale = L.inv_theta;
+  a.e_diag = L.diag;
+  a.e_fixed = M.fixed;
+  return h8_tile_batch_level_launch(a, M.m, l == 0 ? kCoefIso : kCoefQP, smooth ? kModeSmooth : kModeRes, L.P->ox,
+                                    L.P->oy, s);
+}
+
 // Chebyshev smoothing of A x = b on level l (gmg.cu's chebyshev, per-cell interval)
 int bg_chebyshev(const BGmg& M, int l, int deg, bool from_zero, bool need_res, const char* bsum_red,
-                 cudaStream_t s) {
+                 cudaStream_t s, bool* summed = nullptr) {
   const BLevel& L = M.L[l];
   const BVec V = level_mech_vec(L.P);
   int st;
   const double a = 1.0 / 30.0, bm = M.safety;  // interval [lmax/30, safety lmax] relative to lmax
   const double sigma = (bm + a) / (bm - a);
+  const bool one = from_zero && deg == 1;
   if (from_zero) {
-    { note_launch(); bg_first_b_kernel<<<V.n_chunks, kThreads, 0, s>>>(V, L.P->d_cells, L.b, L.invd, L.inv_theta, L.res, L.dvec, L.x, bsum_red, M.guard, M.gstride); }
+    { note_launch(); bg_first_b_kernel<<<V.n_chunks, kThreads, 0, s>>>(V, L.P->d_cells, L.b, L.invd, L.inv_theta, one ? nullptr : L.res, L.dvec, L.x, bsum_red, M.guard, M.gstride); }
+    if (one) return need_res ? bg_level_residual(M, l, L.x, L.res, false, s) : last_launch_status();
   } else {
     if ((st = bg_level_apply(M, l, L.x, L.Ad, s))) return st;
     { note_launch(); bg_first_res_kernel<<<V.n_chunks, kThreads, 0, s>>>(V, L.P->d_cells, L.b, L.Ad, L.invd, L.inv_theta, L.res, L.dvec, L.x, l == 0, L.diag, M.fixed, M.guard, M.gstride); }
@@ -1335,7 +1366,9 @@ int bg_chebyshev(const BGmg& M, int l, int deg, bool from_zero, bool need_res, c
   double rho_old = 1.0 / sigma;
   for (int k = 1; k < deg; ++k) {
     const double rho = 1.0 / (2.0 * sigma - rho_old);
-    if ((st = bg_level_cheb(M, l, cur, oth, rho * rho_old, 2.0 * rho, true, s))) return st;
+    const bool sum = summed && l > 0 && k == deg - 1;
+    if ((st = bg_level_cheb(M, l, cur, oth, rho * rho_old, 2.0 * rho, true, s, sum))) return st;
+    if (sum) *summed = true;
     std::swap(cur, oth);
     rho_old = rho;
   }
@@ -1345,12 +1378,19 @@ int bg_chebyshev(const BGmg& M, int l, int deg, bool from_zero, bool need_res, c
 
 // V-cycle from level l; bsum_red: the pending mean of L.b summed by the parent's restriction;
 // on coarse levels the mean of the result is left pending in L.red for the parent's prolongation
-int bg_vcycle(const BGmg& M, int l, const char* bsum_red, const char** xsum_red, cudaStream_t s) {
+int bg_vcycle(const BGmg& M, int l, const char* bsum_red, const char** xsum_red, const float** xout, float* out,
+              cudaStream_t s) {
   const BLevel& L = M.L[l];
   int st;
   *xsum_red = nullptr;
+  *xout = L.x;
   if (l == M.nlev - 1) {
-    if ((st = bg_chebyshev(M, l, M.deg_coarse, true, false, bsum_red, s))) return st;
+    bool summed = false;
+    if ((st = bg_chebyshev(M, l, M.deg_coarse, true, false, bsum_red, s, &summed))) return st;
+    if (summed) {
+      *xsum_red = L.red;
+      return PHASTB_OK;
+    }
     const BVec Vn = level_node_vec(L.P);
     { note_launch(); bg_mean3_kernel<<<Vn.n_chunks, kThreads, 0, s>>>(Vn, L.P->d_cells, L.x, L.red, M.guard, M.gstride); }
     *xsum_red = L.red;
@@ -1359,11 +1399,19 @@ int bg_vcycle(const BGmg& M, int l, const char* bsum_red, const char** xsum_red,
   if ((st = bg_chebyshev(M, l, M.deg, true, true, bsum_red, s))) return st;
   const BLevel& C = M.L[l + 1];
   const BVec Vcn = level_node_vec(C.P);
-  { note_launch(); bg_restrict_kernel<<<Vcn.n_chunks, kThreads, 0, s>>>(Vcn, L.P->d_cells, C.P->d_cells, L.res, l == 0 ? M.mask : nullptr, C.b, C.red, M.guard, M.gstride); }
+  { note_launch(); bg_restrict_kernel<<<Vcn.n_chunks, kThreads, 0, s>>>(Vcn, L.P->d_cells, C.P->d_cells, L.res, l == 0 && M.deg != 1 ? M.mask : nullptr, C.b, C.red, M.guard, M.gstride); }
   const char* csum = nullptr;
-  if ((st = bg_vcycle(M, l + 1, C.red, &csum, s))) return st;
+  const float* cx = nullptr;
+  if ((st = bg_vcycle(M, l + 1, C.red, &csum, &cx, nullptr, s))) return st;
   const BVec Vfn = level_node_vec(L.P);
-  { note_launch(); bg_prolong_kernel<<<Vfn.n_chunks, kThreads, 0, s>>>(Vfn, L.P->d_cells, C.P->d_cells, C.x, l == 0 ? M.mask : nullptr, L.x, csum, M.guard, M.gstride); }
+  { note_launch(); bg_prolong_kernel<<<Vfn.n_chunks, kThreads, 0, s>>>(Vfn, L.P->d_cells, C.P->d_cells, cx, l == 0 ? M.mask : nullptr, L.x, csum, M.guard, M.gstride); }
+  if (M.deg == 1) {
+    float* y = l == 0 ? out : L.dvec;
+    *xout = y;
+    if ((st = bg_level_residual(M, l, L.x, y, true, s))) return st;
+    if (l > 0) *xsum_red = L.red;
+    return PHASTB_OK;
+  }
   if ((st = bg_chebyshev(M, l, M.deg, false, false, nullptr, s))) return st;
   if (l > 0) {
     const BVec Vn = level_node_vec(L.P);
@@ -1377,9 +1425,10 @@ int bg_vcycle(const BGmg& M, int l, const char* bsum_red, const char** xsum_red,
 int bg_precond(const BGmg& M0, const float* r, float* z, cudaStream_t s) {
   BGmg M = M0;
   M.L[0].b = const_cast<float*>(r);
-  M.L[0].x = z;
+  if (M.deg != 1) M.L[0].x = z;  // (one post-smoothing step writes z itself)
   const char* xs = nullptr;
-  return bg_vcycle(M, 0, nullptr, &xs, s);
+  const float* xo = nullptr;
+  return bg_vcycle(M, 0, nullptr, &xs, &xo, z, s);
 }
 
 // Hierarchy for the current damage field: fine mask and diagonal, coarse moduli and diagonals

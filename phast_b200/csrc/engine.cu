@@ -815,6 +815,32 @@ __global__ void pcg_dir_kernel(int n, PcgWs<T> w) {
     w.p[i] = w.z[i] + beta * w.p[i];
 }
 
+// pcg_rz_kernel (not at the start) and pcg_dir_kernel in one launch, with r . z from the preconditioner: every
+// block derives beta from the same scalars, and the last one to finish stores the state.
+template <typename T>
+__global__ void __launch_bounds__(kThreads) pcg_dir_rz_kernel(int n, PcgWs<T> w, const double* __restrict__ rz_in,
+                                                              int mode) {
+  if (!w.st->active) return;
+  const double RZ = *rz_in, old = w.st->rz;
+  const bool nonfinite = w.st->nonfinite || !isfinite(RZ);
+  const bool breakdown = w.st->breakdown || (mode == PCG_STRICT && !(RZ > 0.0));
+  const double beta = (mode == PCG_STRICT) ? RZ / old : ((old > 0.0) ? RZ / old : 0.0);
+  if (!nonfinite && !breakdown) {
+    const T be = T(beta);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+      w.p[i] = w.z[i] + be * w.p[i];
+  }
+  if (arrive_last(w.counter) && threadIdx.x == 0) {
+    PcgState& st = *w.st;
+    st.nonfinite = nonfinite;
+    st.breakdown = breakdown;
+    st.beta = beta;
+    st.rz = RZ;
+    if (nonfinite || breakdown) st.active = 0;
+    *w.counter = 0u;
+  }
+}
+
 template <typename T>
 int pcg_run(const LinOp<T>& A, int n, const PcgWs<T>& w, const T* b, const T* inv_diag, const Precond<T>* M, T* x,
             double thr, int maxiter, int check_every, PcgMode mode, double, PcgResult* out, cudaStream_t s,
@@ -878,6 +904,11 @@ int pcg_run_thr(const LinOp<T>& A, int n, const PcgWs<T>& w, const T* b, const T
       }
       if (custom) {
         if ((e = M->apply(M->ctx, w.r, w.z, active, s))) return e;
+        if (M->rz_out) {
+          note_launch();
+          pcg_dir_rz_kernel<T><<<G, kThreads, 0, s>>>(n, w, M->rz_out, mode);
+          continue;
+        }
         { note_launch(); pcg_rz_kernel<T><<<G, kThreads, 0, s>>>(n, w, 0, mode); }
       }
       { note_launch(); pcg_dir_kernel<T><<<G, kThreads, 0, s>>>(n, w); }
@@ -893,6 +924,7 @@ int pcg_run_thr(const LinOp<T>& A, int n, const PcgWs<T>& w, const T* b, const T
   if (custom) {
     key_val(key, M->apply);
     key_add(key, M->ctx, M->ctx_bytes);
+    key_val(key, M->rz_out);
   }
   key_val(key, w);
   key_val(key, x);

@@ -107,6 +107,8 @@ struct Precond {
   int (*apply)(const void* ctx, const T* r, T* z, const int* guard, cudaStream_t s);
   const void* ctx;
   size_t ctx_bytes;
+  // Optional: where apply leaves r . z (FP64, device), which spares CG its own reduction.
+  const double* rz_out = nullptr;
 };
 
 // Solves A x = b from x (initial guess held in x, zero allowed).  The caller

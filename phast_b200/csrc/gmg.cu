@@ -251,51 +251,49 @@ __device__ __forceinline__ int fine_of(int i, int n_f, int periodic, bool& ok) {
   return i;
 }
 
-// r_c = R r_f = P^T r_f (full weighting).  The fine vector may carry a mask
-// (rows held at zero are skipped).  With `sum_ws`, the kernel also sums the
-// three components of r_c into sum_ws.out (the coarse level's mean, in the
-// order and grouping of gmg_mean3 over the same grid, so the same bits).
+// r_c = R r_f = P^T r_f (full weighting), one component of a coarse node per thread: three times the threads
+// of a thread per node, neighbours in memory, and all 27 loads in flight (64^3 -> 32^3: 8.3 us with a thread per
+// node and nested loops).  The fine vector may carry a mask (rows held at zero are skipped).  With `want_sum`,
+// the kernel also sums the three components of r_c into sum_ws.out (the coarse level's mean).
 template <typename T>
-__global__ void gmg_restrict(VoxGeom f, VoxGeom c, const T* __restrict__ rf, const uint8_t* __restrict__ mask,
-                             T* __restrict__ rc, RedWs sum_ws, int want_sum, const int* guard) {
+__global__ void __launch_bounds__(kThreads) gmg_restrict(VoxGeom f, VoxGeom c, const T* __restrict__ rf,
+                                                         const uint8_t* __restrict__ mask, T* __restrict__ rc,
+                                                         RedWs sum_ws, int want_sum, const int* guard) {
   if (guard && *guard == 0) return;
   double acc[3] = {0, 0, 0};
-  for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < c.n_red; n += gridDim.x * blockDim.x) {
-    const int I = n % c.rx;
-    const int rem = n / c.rx;
-    const int J = rem % c.ry, K = rem / c.ry;
-    T a0 = 0, a1 = 0, a2 = 0;
-    for (int oz = -1; oz <= 1; ++oz) {
-      bool okz;
-      const int k = fine_of(2 * K + oz, f.nz, f.pz, okz);
-      if (!okz) continue;
-      const T wz = oz == 0 ? T(1) : T(0.5);
-      for (int oy = -1; oy <= 1; ++oy) {
-        bool oky;
-        const int j = fine_of(2 * J + oy, f.ny, f.py, oky);
-        if (!oky) continue;
-        const T wy = oy == 0 ? T(1) : T(0.5);
-        for (int ox = -1; ox <= 1; ++ox) {
-          bool okx;
-          const int i = fine_of(2 * I + ox, f.nx, f.px, okx);
-          if (!okx) continue;
-          const T wgt = (ox == 0 ? T(1) : T(0.5)) * wy * wz;
-          const size_t fn = (size_t)i + (size_t)f.rx * ((size_t)j + (size_t)f.ry * k);
-          const T v0 = (mask && mask[3 * fn + 0]) ? T(0) : rf[3 * fn + 0];
-          const T v1 = (mask && mask[3 * fn + 1]) ? T(0) : rf[3 * fn + 1];
-          const T v2 = (mask && mask[3 * fn + 2]) ? T(0) : rf[3 * fn + 2];
-          a0 += wgt * v0;
-          a1 += wgt * v1;
-          a2 += wgt * v2;
-        }
-      }
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 3 * c.n_red; t += gridDim.x * blockDim.x) {
+    const int n = t / 3, comp = t - 3 * n;
+    const int I = n % c.rx, rem = n / c.rx, J = rem % c.ry, K = rem / c.ry;
+    int i[3], j[3], k[3];
+    bool oi[3], oj[3], ok[3];
+#pragma unroll
+    for (int o = 0; o < 3; ++o) {
+      i[o] = fine_of(2 * I + o - 1, f.nx, f.px, oi[o]);
+      j[o] = fine_of(2 * J + o - 1, f.ny, f.py, oj[o]);
+      k[o] = fine_of(2 * K + o - 1, f.nz, f.pz, ok[o]);
     }
-    rc[3 * (size_t)n + 0] = a0;
-    rc[3 * (size_t)n + 1] = a1;
-    rc[3 * (size_t)n + 2] = a2;
-    acc[0] += double(a0);
-    acc[1] += double(a1);
-    acc[2] += double(a2);
+    T az = T(0);
+#pragma unroll
+    for (int oz = 0; oz < 3; ++oz) {
+      T ay = T(0);
+#pragma unroll
+      for (int oy = 0; oy < 3; ++oy) {
+        T v[3];
+#pragma unroll
+        for (int ox = 0; ox < 3; ++ox) {
+          const bool in = oi[ox] && oj[oy] && ok[oz];
+          const size_t fn =
+              in ? 3 * ((size_t)i[ox] + (size_t)f.rx * ((size_t)j[oy] + (size_t)f.ry * k[oz])) + comp : 0;
+          v[ox] = in && !(mask && mask[fn]) ? __ldg(rf + fn) : T(0);
+        }
+        ay += (oy == 1 ? T(1) : T(0.5)) * (v[1] + T(0.5) * (v[0] + v[2]));
+      }
+      az += (oz == 1 ? T(1) : T(0.5)) * ay;
+    }
+    rc[t] = az;
+    acc[0] += comp == 0 ? double(az) : 0.0;
+    acc[1] += comp == 1 ? double(az) : 0.0;
+    acc[2] += comp == 2 ? double(az) : 0.0;
   }
   if (want_sum) reduce_multi<3>(acc, sum_ws);
 }
@@ -424,9 +422,11 @@ __global__ void gmg_cheb_first_b(int n, T* __restrict__ b, const T* __restrict__
       bi -= m[i % 3];
       b[i] = bi;
     }
-    res[i] = bi;
     const T di = invd[i] * bi * inv_theta;
-    d[i] = di;
+    if (res) {  // (a smoother of one step needs neither)
+      res[i] = bi;
+      d[i] = di;
+    }
     x[i] = di;
   }
 }
@@ -532,7 +532,8 @@ static int coarse_apply(const Gmg<T>& M, const GmgLevel<T>& L, const T* x, T* y,
 
 // One fused Chebyshev step on level l: res -= A din; dout = c1 din + c2 invd res; x += dout.
 template <typename T>
-static int level_cheb(const Gmg<T>& M, int l, const T* din, T* dout, double c1, double c2, cudaStream_t s) {
+static int level_cheb(const Gmg<T>& M, int l, const T* din, T* dout, double c1, double c2, cudaStream_t s,
+                      bool sum_x = false) {
   const GmgLevel<T>& L = M.lv[l];
   TileArgs<T> a = tile_args<T>(L.g, l == 0 ? 0 : 1);
   a.x = din;
@@ -550,6 +551,7 @@ static int level_cheb(const Gmg<T>& M, int l, const T* din, T* dout, double c1, 
     a.mask = M.mask;
     return h8_tile_launch<T>(a, M.mat, M.mat.iso ? kCoefIso : kCoefAniso, kModeCheb, s);
   }
+  if (sum_x) a.ws = M.rw;
   a.lam_q = L.lam;
   a.mu_q = L.mu;
   return h8_tile_launch<T>(a, M.mat, kCoefQP, kModeCheb, s);
@@ -589,18 +591,56 @@ static int pending_mean(const Gmg<T>& M, int l, const T* x, const double** sums,
   return last_launch_status();
 }
 
+// out = b - A x on level l (masked rows zero), or with smooth the one-step smoother
+// out = x + invd (b - A x) / theta (the fine level also writes the E rows' Jacobi step and leaves b . out in
+// M.rw.out[0]; a coarse level leaves out's component sums in M.rw.out).
+template <typename T>
+static int level_residual(const Gmg<T>& M, int l, const T* x, T* out, bool smooth, double inv_theta, cudaStream_t s) {
+  const GmgLevel<T>& L = M.lv[l];
+  TileArgs<T> a = tile_args<T>(L.g, l == 0 ? 0 : 1);
+  a.x = x;
+  a.res = L.b;
+  a.y = out;
+  a.guard = M.guard;
+  a.invd = L.invd;
+  a.c2 = inv_theta;
+  if (smooth) a.ws = M.rw;
+  const int mode = smooth ? kModeSmooth : kModeRes;
+  if (l == 0) {
+    a.slot = M.slot;
+    a.d = M.dfield;
+    a.gq = M.gfield;
+    a.mask = M.mask;
+    a.e_diag = L.diag + 3 * (size_t)L.g.n_red;
+    a.e_fixed = M.fmask + 3 * (size_t)L.g.n_red;
+    return h8_tile_launch<T>(a, M.mat, M.mat.iso ? kCoefIso : kCoefAniso, mode, s);
+  }
+  a.lam_q = L.lam;
+  a.mu_q = L.mu;
+  return h8_tile_launch<T>(a, M.mat, kCoefQP, mode, s);
+}
+
+template <typename T>
+static double cheb_theta(const Gmg<T>& M, int l) {
+  return 0.5 * (M.safety * M.lv[l].lmax + M.lv[l].lmax / 30.0);
+}
+
 // Chebyshev smoothing of A x = b on level l; x starts at zero (from_zero) or at
-// its current value.  With need_res, L.res holds b - A x on exit.
+// its current value.  With need_res, L.res holds b - A x on exit.  With *summed
+// given, it tells whether x's component sums were left in M.rw.out.
 template <typename T>
 static int chebyshev(const Gmg<T>& M, int l, int deg, bool from_zero, bool need_res, const double* bsums,
-                     cudaStream_t s) {
+                     cudaStream_t s, bool* summed = nullptr) {
   const GmgLevel<T>& L = M.lv[l];
   const int n = L.n, G = grid_for(n);
   int st;
   const double bmax = M.safety * L.lmax, amin = L.lmax / 30.0;
   const double theta = 0.5 * (bmax + amin), delta = 0.5 * (bmax - amin), sigma = theta / delta;
+  // one step from zero: the residual is b - A x, without the recurrence's vectors
+  const bool one = from_zero && deg == 1;
   if (from_zero) {
-    { note_launch(); gmg_cheb_first_b<T><<<G, kThreads, 0, s>>>(n, L.b, L.invd, T(1.0 / theta), L.res, L.dvec, L.x, bsums, M.guard); }
+    { note_launch(); gmg_cheb_first_b<T><<<G, kThreads, 0, s>>>(n, L.b, L.invd, T(1.0 / theta), one ? nullptr : L.res, L.dvec, L.x, bsums, M.guard); }
+    if (one) return need_res ? level_residual(M, l, L.x, L.res, false, 0.0, s) : last_launch_status();
   } else {
     if ((st = level_apply(M, l, L.x, L.Ad, s))) return st;
     // on the fine level this is the last pass over the E rows of x: it also
@@ -614,7 +654,9 @@ static int chebyshev(const Gmg<T>& M, int l, int deg, bool from_zero, bool need_
   double rho_old = 1.0 / sigma;
   for (int k = 1; k < deg; ++k) {
     const double rho = 1.0 / (2.0 * sigma - rho_old);
-    if ((st = level_cheb(M, l, cur, oth, rho * rho_old, 2.0 * rho / delta, s))) return st;
+    const bool sum = summed && l > 0 && k == deg - 1;
+    if ((st = level_cheb(M, l, cur, oth, rho * rho_old, 2.0 * rho / delta, s, sum))) return st;
+    if (sum) *summed = true;
     std::swap(cur, oth);
     rho_old = rho;
   }
@@ -625,24 +667,42 @@ static int chebyshev(const Gmg<T>& M, int l, int deg, bool from_zero, bool need_
 
 // V-cycle from level l.  bsums: the pending mean of L.b, summed by the
 // parent's restriction (nullptr on the fine level and on levels without a null
-// space); on coarse levels the mean of the result L.x is left pending
-// (*xsums, see pending_mean) for the parent's prolongation.
+// space); on coarse levels the mean of the result is left pending (*xsums, see
+// pending_mean) for the parent's prolongation.  *xout: where the result is, L.x or,
+// after the fused one-step post-smoothing, `out` (the fine level) or L.dvec.
 template <typename T>
-static int vcycle(const Gmg<T>& M, int l, const double* bsums, const double** xsums, cudaStream_t s) {
+static int vcycle(const Gmg<T>& M, int l, const double* bsums, const double** xsums, const T** xout, T* out,
+                  cudaStream_t s) {
   const GmgLevel<T>& L = M.lv[l];
   int st;
   *xsums = nullptr;
+  *xout = L.x;
+  const bool null_space = L.g.px && L.g.py && L.g.pz;
   if (l == M.nlev - 1) {
-    if ((st = chebyshev(M, l, M.deg_coarse, true, false, bsums, s))) return st;
+    bool summed = false;
+    if ((st = chebyshev(M, l, M.deg_coarse, true, false, bsums, s, null_space ? &summed : nullptr))) return st;
+    if (summed) {
+      *xsums = M.rw.out;
+      return PHASTB_OK;
+    }
     return pending_mean(M, l, L.x, xsums, s);
   }
   if ((st = chebyshev(M, l, M.deg, true, true, bsums, s))) return st;
   const GmgLevel<T>& C = M.lv[l + 1];
   const int cper = C.g.px && C.g.py && C.g.pz;  // the coarse level has a null space: sum its mean
-  { note_launch(); gmg_restrict<T><<<grid_for(C.g.n_red), kThreads, 0, s>>>(L.g, C.g, L.res, l == 0 ? M.mask : nullptr, C.b, M.rw, cper, M.guard); }
+  const uint8_t* rmask = l == 0 && M.deg != 1 ? M.mask : nullptr;  // (one step: the residual's masked rows are zero)
+  { note_launch(); gmg_restrict<T><<<grid_for(3LL * C.g.n_red), kThreads, 0, s>>>(L.g, C.g, L.res, rmask, C.b, M.rw, cper, M.guard); }
   const double* csums = nullptr;
-  if ((st = vcycle(M, l + 1, cper ? M.rw.out : nullptr, &csums, s))) return st;
-  { note_launch(); gmg_prolong_add<T><<<grid_for(L.g.n_red), kThreads, 0, s>>>(L.g, C.g, C.x, l == 0 ? M.mask : nullptr, L.x, csums, M.guard); }
+  const T* cx = nullptr;
+  if ((st = vcycle<T>(M, l + 1, cper ? M.rw.out : nullptr, &csums, &cx, nullptr, s))) return st;
+  { note_launch(); gmg_prolong_add<T><<<grid_for(L.g.n_red), kThreads, 0, s>>>(L.g, C.g, cx, l == 0 ? M.mask : nullptr, L.x, csums, M.guard); }
+  if (M.deg == 1) {
+    T* y = l == 0 ? out : L.dvec;
+    *xout = y;
+    if ((st = level_residual(M, l, L.x, y, true, 1.0 / cheb_theta(M, l), s))) return st;
+    if (l > 0 && null_space) *xsums = M.rw.out;
+    return PHASTB_OK;
+  }
   if ((st = chebyshev(M, l, M.deg, false, false, nullptr, s))) return st;
   if (l > 0 && (st = pending_mean(M, l, L.x, xsums, s))) return st;
   return last_launch_status();
@@ -792,6 +852,12 @@ static int gmg_setup(Gmg<T>& M, const VoxMat<T>& mat, const uint8_t* slot, const
   return PHASTB_OK;
 }
 
+// Whether the V-cycle's last kernel leaves r . z in M.rw.out[0] (one post-smoothing step).
+template <typename T>
+static bool gmg_fused_rz(const Gmg<T>& M) {
+  return M.deg == 1 && M.nlev > 1;
+}
+
 // z = M^-1 r: V-cycle on the fluctuation rows, Jacobi on the free E rows.
 template <typename T>
 static int gmg_precond_apply(const void* ctx, const T* r, T* z, const int* guard, cudaStream_t s) {
@@ -801,12 +867,14 @@ static int gmg_precond_apply(const void* ctx, const T* r, T* z, const int* guard
   Gmg<T> Mg = M;
   Mg.guard = guard;
   // the fine level reads its right-hand side from r (never written there: the
-  // fine level has no pending mean) and builds its iterate directly in z
+  // fine level has no pending mean); one post-smoothing step writes z, more build
+  // the iterate in z
   Mg.lv[0].b = const_cast<T*>(r);
-  Mg.lv[0].x = z;
+  if (!gmg_fused_rz(M)) Mg.lv[0].x = z;
   const double* xsums = nullptr;
-  // the fine level's post-smoothing also writes z's E rows (gmg_cheb_first_res)
-  if ((st = vcycle(Mg, 0, nullptr, &xsums, s))) return st;
+  const T* xo = nullptr;
+  // the fine level's post-smoothing also writes z's E rows
+  if ((st = vcycle<T>(Mg, 0, nullptr, &xsums, &xo, z, s))) return st;
   return last_launch_status();
 }
 
@@ -1061,7 +1129,8 @@ static int mech_solve_ex_impl(const phastb_voxel_grid* g, const phastb_voxel_mat
       if ((st = gmg_setup<double>(L.g64, m64, slot, dd, fixed, o->smooth_degree, o->coarse_degree, o->power_iters,
                                   o->lmax_safety, lmax_io, s, gg)))
         return st;
-      Precond<double> M{gmg_precond_apply<double>, &L.g64, sizeof(L.g64)};
+      Precond<double> M{gmg_precond_apply<double>, &L.g64, sizeof(L.g64),
+                        gmg_fused_rz(L.g64) ? L.g64.rw.out : nullptr};
       if ((st = cuda_status(cudaMemcpyAsync(L.x64, x_out, sizeof(double) * n, cudaMemcpyDeviceToDevice, s))))
         return st;
       if ((st = pcg_run<double>(A64, n, L.w64, L.bf, nullptr, &M, L.x64, thr, maxiter, gmg_check(), PCG_FREEZE, 0.0,
@@ -1109,7 +1178,7 @@ static int mech_solve_ex_impl(const phastb_voxel_grid* g, const phastb_voxel_mat
   MechOpT<float> free32{v, m32, slot, d32, fixed, scratch32, g32};
   LinOp<float> A32{mech_op_t<float>, &free32, sizeof(free32), mech_op_dot_t<float>,
                    h8_apply_dot_slot(v, 4, scratch32)};
-  Precond<float> M32{gmg_precond_apply<float>, &L.g32, sizeof(L.g32)};
+  Precond<float> M32{gmg_precond_apply<float>, &L.g32, sizeof(L.g32), gmg_fused_rz(L.g32) ? L.g32.rw.out : nullptr};
   int total = 0, converged = 0;
   double rn = bn;
   for (int k = 0; k < o->max_refine && total < maxiter; ++k) {

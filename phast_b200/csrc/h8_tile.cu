@@ -139,9 +139,10 @@ __device__ __forceinline__ void tile_body(const TileArgs<T>& a, const VoxMat<T>&
   constexpr bool DOT = MODE == kModeDot, ENERGY = MODE == kModeEnergy, CHEB = MODE == kModeCheb;
   // E rows (macro strain) exist on the fine operator; a Chebyshev step and a
   // nodal-block action leave them alone (masked)
-  constexpr bool NODAL = MODE == kModeNodal;
-  constexpr bool EROWS = SLOT && !CHEB && !NODAL;
-  constexpr bool RED = EROWS || DOT || ENERGY;
+  constexpr bool NODAL = MODE == kModeNodal, RES = MODE == kModeRes, SMOOTH = MODE == kModeSmooth;
+  constexpr bool EROWS = SLOT && !CHEB && !NODAL && !RES && !SMOOTH;
+  constexpr bool RED = EROWS || DOT || ENERGY || SMOOTH;
+  constexpr bool EPI = CHEB || RES || SMOOTH;  // the epilogue reads vectors of the owned nodes
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const VoxGeom& g = a.g;
   if (NODAL && vb == 0 && threadIdx.x < 6 && a.y) a.y[3 * (size_t)g.n_red + threadIdx.x] = T(0);
@@ -161,9 +162,9 @@ __device__ __forceinline__ void tile_body(const TileArgs<T>& a, const VoxMat<T>&
   T* nb = reinterpret_cast<T*>(sbase);  // [3 buffers][nt][4 fields] (without TMA)
   size_t off_face = 0, off_qp = 0, off_cheb = 0;
   if (TMA) {
-    tile_layout_tma<T>(ox, oy, COEF == kCoefQP, CHEB, &off_face, &off_qp, &off_cheb);
+    tile_layout_tma<T>(ox, oy, COEF == kCoefQP, EPI, &off_face, &off_qp, &off_cheb);
   } else {
-    tile_layout<T>(ox, oy, COEF == kCoefQP, CHEB, &off_qp, &off_cheb);
+    tile_layout<T>(ox, oy, COEF == kCoefQP, EPI, &off_qp, &off_cheb);
     off_face = sizeof(T) * 12 * (size_t)nt;
   }
   T* FC = reinterpret_cast<T*>(sbase + off_face);  // corner forces of one node layer, [4 corners][3 comps][exy]
@@ -193,6 +194,16 @@ __device__ __forceinline__ void tile_body(const TileArgs<T>& a, const VoxMat<T>&
   const T c1 = T(a.c1), c2 = T(a.c2);
   // macro strain, read from shared memory where it is used (six registers fewer per thread); a Chebyshev
   // step smooths the nodal block only (E rows masked).  The first barrier of the march orders the store.
+  // All six E rows masked (a cell under full macro-strain control): CG's action does not form their sums, and
+  // its reduction shrinks from eight values to the dot product.
+  bool e_live = EROWS;
+  if constexpr (EROWS && DOT) {
+    if (a.mask) {
+      const uint8_t* em = a.mask + 3 * (size_t)g.n_red;
+      e_live = !(__ldg(em) && __ldg(em + 1) && __ldg(em + 2) && __ldg(em + 3) && __ldg(em + 4) && __ldg(em + 5));
+      if (!e_live && vb == 0 && threadIdx.x < 6 && a.y) a.y[3 * (size_t)g.n_red + threadIdx.x] = T(0);
+    }
+  }
   __shared__ T E6[6];
   if (EROWS && tid < 6) E6[tid] = __ldg(x + 3 * (size_t)g.n_red + tid);
   const int tiles_x = (g.rx + ox - 1) / ox, tiles_y = (g.ry + oy - 1) / oy;
@@ -307,6 +318,8 @@ __device__ __forceinline__ void tile_body(const TileArgs<T>& a, const VoxMat<T>&
     }
   };
   double accd[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  // a coarse level's last Chebyshev step also sums x's components (a reduction workspace is given then)
+  const bool sum_x = CHEB && !SLOT && a.ws.counter != nullptr;
   const size_t plane_n = (size_t)g.rx * g.ry, plane_e = (size_t)g.nx * g.ny;
 
   for (int tile = vb; tile < n_tiles; tile += vgrid) {
@@ -374,17 +387,18 @@ __device__ __forceinline__ void tile_body(const TileArgs<T>& a, const VoxMat<T>&
         }
       }
     };
-    // kModeCheb: cp.async of (res, invd, xs) of the owned node in node layer kn into buffer `buf`
+    // kModeCheb: cp.async of (res, invd, xs) of the owned node in node layer kn into buffer `buf` (kModeSmooth:
+    // res and invd, kModeRes: res)
     auto stage_cheb = [&](int kn, int buf) {
-      if constexpr (CHEB) {
+      if constexpr (EPI) {
         if (no >= 0) {
           const size_t n3 = 3 * (plane_n * kn + no);
           T* dst = CS + (size_t)buf * 9 * oxy + tid;
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
             cp_async_word(dst + c * oxy, a.res + n3 + c);
-            cp_async_word(dst + (3 + c) * oxy, a.invd + n3 + c);
-            cp_async_word(dst + (6 + c) * oxy, a.xs + n3 + c);
+            if (!RES) cp_async_word(dst + (3 + c) * oxy, a.invd + n3 + c);
+            if (CHEB) cp_async_word(dst + (6 + c) * oxy, a.xs + n3 + c);
           }
         }
       }
@@ -434,7 +448,7 @@ __device__ __forceinline__ void tile_body(const TileArgs<T>& a, const VoxMat<T>&
       }
       __syncthreads();
       // every thread is done with buffer (kk + 2) % 3 (node layer ke - 1): refill it with layer ke + 2
-      if constexpr (CHEB) {
+      if constexpr (EPI) {
         if (kk >= 1) stage_cheb(ke, kk & 1);
         cp_async_commit();
       }
@@ -602,7 +616,7 @@ __device__ __forceinline__ void tile_body(const TileArgs<T>& a, const VoxMat<T>&
             const T m0 = Pz[c][0][1] - Pz[c][0][0], m1 = Pz[c][1][1] - Pz[c][1][0];
             const T T0 = p0 + p1, TY = p1 - p0, TX = m0 + m1, TXY = m1 - m0;
             const T sx = Sx[c][0] + Sx[c][1], sy = Sy[c][0] + Sy[c][1];
-            if (EROWS && own) {
+            if (EROWS && own && e_live) {
               if (c == 0) {
                 tacc[0] += sx;
                 tacc[5] += sy;
@@ -645,7 +659,7 @@ __device__ __forceinline__ void tile_body(const TileArgs<T>& a, const VoxMat<T>&
       }
       if (kk == 0) continue;  // the first element layer only fills pend
       __syncthreads();
-      if constexpr (CHEB) cp_async_wait<1>();  // this thread's (res, invd, xs) of node layer ke
+      if constexpr (EPI) cp_async_wait<1>();  // this thread's (res, invd, xs) of node layer ke
       // ---- node phase: node layer ke, the four columns that meet at the node
       if (no >= 0) {
         const int e11 = (ni + 1) + ex * (nj + 1), e01 = ni + ex * (nj + 1);
@@ -664,7 +678,23 @@ __device__ __forceinline__ void tile_body(const TileArgs<T>& a, const VoxMat<T>&
               a.res[i] = r;
               const T dn = c1 * xin + c2 * cs[(3 + c) * oxy] * r;
               a.d_out[i] = dn;
-              a.xs[i] = cs[(6 + c) * oxy] + dn;
+              const T xn = cs[(6 + c) * oxy] + dn;
+              a.xs[i] = xn;
+              if (!SLOT && sum_x) accd[c] += double(xn);
+            } else if (RES || SMOOTH) {
+              const T b = CS[(size_t)(kk & 1) * 9 * oxy + tid + c * oxy];
+              T r = b - v;
+              if (RES) {
+                if (mk_cur & (1 << c)) r = T(0);
+                a.y[i] = r;
+              } else {
+                const T z = xin + c2 * CS[(size_t)(kk & 1) * 9 * oxy + tid + (3 + c) * oxy] * r;
+                a.y[i] = z;
+                if (SLOT)
+                  accd[0] += double(b) * double(z);
+                else
+                  accd[c] += double(z);
+              }
             } else {
               if (a.y) a.y[i] = v;
               if (DOT) tacc[kOutDot] += xin * v;
@@ -673,7 +703,7 @@ __device__ __forceinline__ void tile_body(const TileArgs<T>& a, const VoxMat<T>&
         }
       }
     }
-    if (RED) {
+    if (RED && !SMOOTH) {
 #pragma unroll
       for (int k = 0; k < 8; ++k) accd[k] += double(tacc[k]);
     }
@@ -688,21 +718,52 @@ __device__ __forceinline__ void tile_body(const TileArgs<T>& a, const VoxMat<T>&
     for (int k = 0; k < 8; ++k) accd[k] = NAN;
   }
 
-  if constexpr (RED) {
-    constexpr int NK = DOT ? 8 : (ENERGY ? 7 : 6);
+  // Sums of v[0..NK) over the grid's (or cell's) blocks: the last block to arrive folds the partials.
+  auto grid_sum = [&](auto nk, double* v, auto finish) {
+    constexpr int NK = decltype(nk)::value;
     __shared__ double sh[32 * NK];
-    double v[NK];
+    double b[NK];
 #pragma unroll
-    for (int k = 0; k < NK; ++k) v[k] = accd[k];
-    block_sum_multi<NK>(v, sh);
+    for (int k = 0; k < NK; ++k) b[k] = v[k];
+    block_sum_multi<NK>(b, sh);
     if (tid == 0) {
 #pragma unroll
-      for (int k = 0; k < NK; ++k) a.ws.part[k * kMaxPartials + vb] = v[k];
+      for (int k = 0; k < NK; ++k) a.ws.part[k * kMaxPartials + vb] = b[k];
     }
     if (arrive_last_n(a.ws.counter, vgrid)) {
       double f[NK];
       fold_sum_multi<NK>(a.ws.part, kMaxPartials, vgrid, f, sh);
       if (tid == 0) {
+        finish(f);
+        *a.ws.counter = 0u;
+      }
+    }
+  };
+  if constexpr (CHEB && !SLOT) {
+    if (sum_x)
+      grid_sum(std::integral_constant<int, 3>{}, accd, [&](const double* f) {
+        for (int k = 0; k < 3; ++k) a.ws.out[k] = f[k];
+      });
+  } else if constexpr (SMOOTH) {
+    if constexpr (SLOT) {
+      if (vb == 0 && tid == 0) {  // the E rows' Jacobi step and their share of res . y
+        const size_t e = 3 * (size_t)g.n_red;
+        for (int k = 0; k < 6; ++k) {
+          const T z = a.e_fixed[k] ? T(0) : a.res[e + k] / a.e_diag[k];
+          a.y[e + k] = z;
+          accd[0] += double(a.res[e + k]) * double(z);
+        }
+      }
+      grid_sum(std::integral_constant<int, 1>{}, accd, [&](const double* f) { a.ws.out[0] = f[0]; });
+    } else {
+      grid_sum(std::integral_constant<int, 3>{}, accd, [&](const double* f) {
+        for (int k = 0; k < 3; ++k) a.ws.out[k] = f[k];
+      });
+    }
+  } else if constexpr (RED) {
+    constexpr int NK = DOT ? 8 : (ENERGY ? 7 : 6);
+    if (e_live || !EROWS) {
+      grid_sum(std::integral_constant<int, NK>{}, accd, [&](const double* f) {
         double dot_e = 0.0;
 #pragma unroll
         for (int k = 0; k < NK; ++k) {
@@ -719,8 +780,9 @@ __device__ __forceinline__ void tile_body(const TileArgs<T>& a, const VoxMat<T>&
             a.ws.out[k] = t + dot_e;
           }
         }
-        *a.ws.counter = 0u;
-      }
+      });
+    } else if constexpr (DOT) {
+      grid_sum(std::integral_constant<int, 1>{}, accd + kOutDot, [&](const double* f) { a.ws.out[kOutDot] = f[0]; });
     }
   }
 }
@@ -1102,6 +1164,9 @@ __global__ void __launch_bounds__(kTileMaxThreads, 2) h8_damage_pcg_kernel(DTile
 
 namespace {
 
+// Modes whose epilogue stages vectors of the owned nodes (see tile_layout's cheb).
+constexpr bool mode_epi(int mode) { return mode == kModeCheb || mode == kModeRes || mode == kModeSmooth; }
+
 std::mutex g_shape_mu;
 std::map<std::tuple<int, int, int, int, int, int, int, int>, TileShape> g_shapes;
 
@@ -1285,9 +1350,9 @@ int launch_variant_t(const TileArgs<T>& a, const VoxMat<T>& m, cudaStream_t s, c
                      const CUtensorMap& md) {
   auto kern = h8_tile_kernel<T, COEF, MODE, OX, OY, TMA>;
   size_t off_face = 0, off_qp = 0, off_cheb = 0;
-  const size_t smem = TMA ? tile_layout_tma<T>(a.ts.ox, a.ts.oy, COEF == kCoefQP, MODE == kModeCheb, &off_face,
+  const size_t smem = TMA ? tile_layout_tma<T>(a.ts.ox, a.ts.oy, COEF == kCoefQP, mode_epi(MODE), &off_face,
                                                &off_qp, &off_cheb)
-                          : tile_layout<T>(a.ts.ox, a.ts.oy, COEF == kCoefQP, MODE == kModeCheb, &off_qp, &off_cheb);
+                          : tile_layout<T>(a.ts.ox, a.ts.oy, COEF == kCoefQP, mode_epi(MODE), &off_qp, &off_cheb);
   const int threads = tile_threads(a.ts);
   static std::mutex mu;
   static size_t smem_set = 0;
@@ -1411,6 +1476,12 @@ int dispatch(const TileArgs<T>& a, const VoxMat<T>& m, int coef, int mode, cudaS
     case kCoefIso * 8 + kModeEnergy: return launch_variant<T, kCoefIso, kModeEnergy, 0, 0>(a, m, s);
     case kCoefIso * 8 + kModeCheb: return by_shape<T, kCoefIso, kModeCheb>(a, m, s);
     case kCoefIso * 8 + kModeNodal: return by_shape<T, kCoefIso, kModeNodal>(a, m, s);
+    case kCoefIso * 8 + kModeRes: return by_shape<T, kCoefIso, kModeRes>(a, m, s);
+    case kCoefIso * 8 + kModeSmooth: return by_shape<T, kCoefIso, kModeSmooth>(a, m, s);
+    case kCoefAniso * 8 + kModeRes: return launch_variant<T, kCoefAniso, kModeRes, 0, 0>(a, m, s);
+    case kCoefAniso * 8 + kModeSmooth: return launch_variant<T, kCoefAniso, kModeSmooth, 0, 0>(a, m, s);
+    case kCoefQP * 8 + kModeRes: return by_shape<T, kCoefQP, kModeRes>(a, m, s);
+    case kCoefQP * 8 + kModeSmooth: return by_shape<T, kCoefQP, kModeSmooth>(a, m, s);
     case kCoefAniso * 8 + kModeApply: return launch_variant<T, kCoefAniso, kModeApply, 0, 0>(a, m, s);
     case kCoefAniso * 8 + kModeDot: return launch_variant<T, kCoefAniso, kModeDot, 0, 0>(a, m, s);
     case kCoefAniso * 8 + kModeEnergy: return launch_variant<T, kCoefAniso, kModeEnergy, 0, 0>(a, m, s);
@@ -1814,7 +1885,10 @@ __global__ void __launch_bounds__(TileBounds<T, OX, OY>::threads, TileBounds<T, 
     a.d_out = b.d_out ? b.d_out + c.mech_off : nullptr;
     a.c1 = b.c1;
     a.c2 = b.c2 * (b.c2_scale ? b.c2_scale[wk.x] : 1.0);
-    a.ws = red_ws(b.ws + (size_t)wk.x * red_ws_bytes());
+    const long long e6 = c.mech_off + 3LL * c.g.n_red;
+    a.e_diag = b.e_diag ? b.e_diag + e6 : nullptr;
+    a.e_fixed = b.e_fixed ? b.e_fixed + e6 : nullptr;
+    a.ws = b.ws ? red_ws(b.ws + (size_t)wk.x * red_ws_bytes()) : RedWs{nullptr, nullptr, nullptr};
     a.guard = b.guard ? b.guard + (size_t)wk.x * b.guard_stride : nullptr;
     a.k = batch_k<T>(c);
     sa = a;
@@ -1890,7 +1964,7 @@ template <int COEF, int MODE, int OX, int OY>
 int tile_batch_level_variant(const TileBatchArgs<float>& b, const VoxMat<float>& m, cudaStream_t s) {
   auto kern = h8_tile_batch_kernel<float, MODE, OX, OY, COEF>;
   size_t oq = 0, oc = 0;
-  const size_t smem = tile_layout<float>(OX, OY, COEF == kCoefQP, MODE == kModeCheb, &oq, &oc);
+  const size_t smem = tile_layout<float>(OX, OY, COEF == kCoefQP, mode_epi(MODE), &oq, &oc);
   int st = batch_smem_attr(kern, smem);
   if (st) return st;
   const int threads = ((OX + 1) * (OY + 1) + 31) / 32 * 32;
@@ -1931,14 +2005,20 @@ int h8_tile_batch_level_launch(const TileBatchArgs<float>& b, const VoxMat<float
   if (coef == kCoefIso && !m.iso) return PHASTB_UNSUPPORTED;
   if (coef == kCoefIso && ox == 16 && oy == 8) {
     if (mode == kModeCheb) return tile_batch_level_variant<kCoefIso, kModeCheb, 16, 8>(b, m, s);
+    if (mode == kModeRes) return tile_batch_level_variant<kCoefIso, kModeRes, 16, 8>(b, m, s);
+    if (mode == kModeSmooth) return tile_batch_level_variant<kCoefIso, kModeSmooth, 16, 8>(b, m, s);
     if (mode == kModeNodal) return tile_batch_level_variant<kCoefIso, kModeNodal, 16, 8>(b, m, s);
   }
   if (coef == kCoefIso && ox == 8 && oy == 8) {
     if (mode == kModeCheb) return tile_batch_level_variant<kCoefIso, kModeCheb, 8, 8>(b, m, s);
+    if (mode == kModeRes) return tile_batch_level_variant<kCoefIso, kModeRes, 8, 8>(b, m, s);
+    if (mode == kModeSmooth) return tile_batch_level_variant<kCoefIso, kModeSmooth, 8, 8>(b, m, s);
     if (mode == kModeNodal) return tile_batch_level_variant<kCoefIso, kModeNodal, 8, 8>(b, m, s);
   }
   if (coef == kCoefQP && ox == 8 && oy == 8) {
     if (mode == kModeCheb) return tile_batch_level_variant<kCoefQP, kModeCheb, 8, 8>(b, m, s);
+    if (mode == kModeRes) return tile_batch_level_variant<kCoefQP, kModeRes, 8, 8>(b, m, s);
+    if (mode == kModeSmooth) return tile_batch_level_variant<kCoefQP, kModeSmooth, 8, 8>(b, m, s);
     if (mode == kModeApply) return tile_batch_level_variant<kCoefQP, kModeApply, 8, 8>(b, m, s);
   }
   return PHASTB_ERR_ARG;

@@ -119,8 +119,14 @@ enum ApplyOut { kOutE = 0, kOutEnergy = 6, kOutDot = 7, kApplyOuts = 8 };
 enum TileCoef { kCoefIso = 0, kCoefAniso = 1, kCoefQP = 2 };
 // Node epilogue: y = A x; y and x . y; y and the energy; one Chebyshev step;
 // y = A x on the nodal block only (the macro-strain E rows of x are not read,
-// those of y are set to zero: a smoother's residual with the E rows masked).
-enum TileMode { kModeApply = 0, kModeDot = 1, kModeEnergy = 2, kModeCheb = 3, kModeNodal = 4 };
+// those of y are set to zero: a smoother's residual with the E rows masked);
+// y = res - A x on the nodal block (masked rows zero); one smoothing step from x,
+// y = x + c2 invd (res - A x) on the nodal block, with, on the fine level, the E
+// rows' Jacobi step y_E = fixed ? 0 : res_E / e_diag and res . y at ws.out[0], on a
+// coarse level the component sums of y at ws.out[0..2].
+enum TileMode {
+  kModeApply = 0, kModeDot = 1, kModeEnergy = 2, kModeCheb = 3, kModeNodal = 4, kModeRes = 5, kModeSmooth = 6
+};
 
 // Gauss-point constants of the action: N1 weights with the 1/h of each axis
 // folded in (the last interpolation stage of a derivative applies them).
@@ -163,6 +169,8 @@ struct TileArgs {
   T* xs;
   T* d_out;
   double c1, c2;
+  const T* e_diag;         // kModeSmooth, fine level: diagonal and mask of the E rows (six entries)
+  const uint8_t* e_fixed;
   RedWs ws;
   const int* guard;
   TileK<T> k;
@@ -287,6 +295,8 @@ struct TileBatchArgs {
   T* d_out;
   double c1, c2;
   const double* c2_scale;
+  const T* e_diag;  // kModeSmooth, fine level: laid out like x (the E rows are read)
+  const uint8_t* e_fixed;
 };
 
 // One multigrid-level launch of the batch: kCoefIso (the fine level: slots and g(d)) or kCoefQP
