@@ -210,6 +210,7 @@ PFCZM_ENERGY_WORDS = 4 + MAX_SLOTS
 
 _lock = threading.Lock()
 _lib = None
+_fns = {}  # entry points by name, filled by load()
 
 
 def load():
@@ -226,6 +227,7 @@ def load():
                 fn = getattr(lib, name)
                 fn.restype = res
                 fn.argtypes = args
+                _fns[name] = fn
             _lib = lib
         return _lib
 
@@ -247,16 +249,20 @@ def check(status, fn):
     raise PhastbError(fn, status)
 
 
-def call(name, *args):
-    """Call an entry point and raise on any non-OK status."""
-    st = getattr(load(), name)(*args)
-    check(st, name)
-    return st
-
-
 def raw(name, *args):
     """Call an entry point and return its status (solvers report convergence this way)."""
-    return getattr(load(), name)(*args)
+    fn = _fns.get(name)
+    if fn is None:
+        fn = getattr(load(), name)
+    return fn(*args)
+
+
+def call(name, *args):
+    """Call an entry point and raise on any non-OK status."""
+    st = raw(name, *args)
+    if st != OK:
+        check(st, name)
+    return st
 
 
 def ptr(t):
@@ -265,13 +271,21 @@ def ptr(t):
         return None
     if not t.is_contiguous():
         raise ValueError("phast_b200 kernels need contiguous tensors")
-    if t.data_ptr() % 16:
+    p = t.data_ptr()
+    if p % 16:
         raise ValueError("phast_b200 kernels need 16-byte aligned tensors (vectorised loads)")
-    return C.c_void_p(t.data_ptr())
+    return vp(p)
+
+
+# the current stream's handle without building a Stream object (a microsecond of every call)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
 def stream(device=None):
-    return C.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    if _raw_stream is not None:
+        index = torch.device(device).index if device is not None else None
+        return vp(_raw_stream(torch.cuda.current_device() if index is None else index))
+    return vp(torch.cuda.current_stream(device).cuda_stream)
 
 
 def require_cuda(t, name="tensor"):

@@ -246,10 +246,10 @@ class PeriodicVoxelPhaseFieldOperator:
 
     def scratch(self, dtype=torch.float64):
         code = _lib.F64 if dtype == torch.float64 else _lib.F32
-        nbytes = _lib.load().phastb_h8_scratch_bytes(self.vgrid, code)
         attr = "_scratch64" if code == _lib.F64 else "_scratch32"
         buf = getattr(self, attr)
-        if buf is None or buf.numel() < nbytes:
+        if buf is None:  # (its size depends on the grid alone)
+            nbytes = _lib.load().phastb_h8_scratch_bytes(self.vgrid, code)
             buf = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
             setattr(self, attr, buf)
         return C.c_void_p(buf.data_ptr())

@@ -112,21 +112,31 @@ class BoundaryConditions:
         self.pf_dirichlet_bcs.append((idx, float(value)))
         return self
 
+    def _nodes_on_device(self, idx):
+        """The node list on the device; indices are checked here, on the host (a device-side check aborts)."""
+        if idx.numel() and not (-self.n_nodes <= int(idx.min()) and int(idx.max()) < self.n_nodes):
+            raise IndexError(f"boundary node index out of range for {self.n_nodes} nodes")
+        return idx.to(self.device)
+
+    # the masks are filled where they are used: the node lists are short, the nodal arrays are not (400 x 160:
+    # 1.2 MB through pageable copies in every explicit step before)
     def get_masks_and_values(self):
-        mask = torch.zeros(self.n_nodes, 2, dtype=torch.bool)
-        vals = torch.zeros(self.n_nodes, 2, dtype=self.dtype)
+        mask = torch.zeros(self.n_nodes, 2, dtype=torch.bool, device=self.device)
+        vals = torch.zeros(self.n_nodes, 2, dtype=self.dtype, device=self.device)
         for idx, c, v in self.bcs:
-            mask[idx, c] = True
-            vals[idx, c] = v * self.load_factor
-        return mask.to(self.device), vals.to(self.device)
+            where = self._nodes_on_device(idx)
+            mask[where, c] = True
+            vals[where, c] = v * self.load_factor
+        return mask, vals
 
     def get_pf_dirichlet_mask_values(self):
-        mask = torch.zeros(self.n_nodes, dtype=torch.bool)
-        vals = torch.zeros(self.n_nodes, dtype=self.dtype)
+        mask = torch.zeros(self.n_nodes, dtype=torch.bool, device=self.device)
+        vals = torch.zeros(self.n_nodes, dtype=self.dtype, device=self.device)
         for idx, v in self.pf_dirichlet_bcs:
-            mask[idx] = True
-            vals[idx] = v
-        return mask.to(self.device), vals.to(self.device)
+            where = self._nodes_on_device(idx)
+            mask[where] = True
+            vals[where] = v
+        return mask, vals
 
 
 class AndersonAccelerator:
