@@ -1141,8 +1141,12 @@ static int mech_solve_ex_impl(const phastb_voxel_grid* g, const phastb_voxel_mat
       { note_launch(); gmg_invert<double><<<G, kThreads, 0, s>>>(n, L.r64, fixed, L.r64); }
       if ((st = cuda_status(cudaMemcpyAsync(L.x64, x_out, sizeof(double) * n, cudaMemcpyDeviceToDevice, s))))
         return st;
+      const PcgLoop loop = [&](int mi) {  // see mech_solve_impl
+        return h8_mech_brick_pcg(v, m64, slot, gg, dd, fixed, L.w64, L.scratch64,
+                                 align_up(24 * sizeof(double) * (size_t)v.n_elem), L.x64, L.r64, mi, PCG_FREEZE, s);
+      };
       if ((st = pcg_run<double>(A64, n, L.w64, L.bf, L.r64, nullptr, L.x64, thr, maxiter, check_every, PCG_FREEZE,
-                                0.0, &pr, s)))
+                                0.0, &pr, s, &loop)))
         return st;
     }
     if ((st = cuda_status(cudaMemcpyAsync(x_out, L.x64, sizeof(double) * n, cudaMemcpyDeviceToDevice, s))))

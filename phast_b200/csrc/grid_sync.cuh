@@ -86,7 +86,7 @@ struct GridSync {
 template <int K, int M, int kT, class Overlap>
 __device__ __forceinline__ bool grid_reduce(double (&v)[K + M], GridSync& g, Overlap overlap) {
   constexpr int N = K + M, kW = kT / 32, kFold = (kGridBlocks + 31) / 32;
-  static_assert(N <= kGridValues && N * kFold <= kW && kW <= 32, "kFold warps per value, one lane per warp's share");
+  static_assert(N <= kGridValues && N < kW && kW <= 32, "a warp per value and one to spare, a lane per warp's share");
   __shared__ double s_warp[N][kW];
   __shared__ double s_fold[N][kFold];
   __shared__ double s_out[N];
@@ -124,9 +124,9 @@ __device__ __forceinline__ bool grid_reduce(double (&v)[K + M], GridSync& g, Ove
     }
   }
   if (G > 1 && !direct && root) {
-    // kFold warps per value, one word per thread
-    const int k = w / kFold, part = w - k * kFold;
-    if (k < N) {
+    // kFold parts per value, one word per thread
+    for (int j = w; j < N * kFold; j += kW) {
+      const int k = j / kFold, part = j - k * kFold;
       const bool sum = k < K;
       const int b = 32 * part + l;
       double t = sum ? 0.0 : INFINITY;

@@ -1,6 +1,6 @@
 // Tiled z-marching voxel H8 elastic action (see h8_tile.cuh).
 #include "h8_tile.cuh"
-#include "h8_march.cuh"
+#include "h8_elastic.cuh"
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include "engine.cuh"
@@ -91,22 +91,6 @@ __device__ __forceinline__ void get4(const double* p, double (&v)[4]) {
   v[2] = r.x;
   v[3] = r.y;
 }
-
-// One node layer as an element sees it: the four corner values of u~ in the Haar basis of the
-// face (x difference X, y difference Y, mixed difference XY; the sum M as four times the first
-// corner's value V plus differences R, so that only differences of nodal values are ever rounded),
-// and 1 - d at the face's four Gauss positions o[qx + 2 qy] (interpolated in x and y).
-template <typename T>
-struct Face {
-  T V[3], R[3], X[3], Y[3], XY[3];
-  T o[4];
-};
-
-// The element's share of a node layer's forces, in the same Haar basis.
-template <typename T>
-struct FaceForce {
-  T M[3], X[3], Y[3], XY[3];
-};
 
 }  // namespace
 
@@ -238,23 +222,8 @@ __device__ __forceinline__ void tile_body(const TileArgs<T>& a, const VoxMat<T>&
         get4(nb + 4 * (nt * buf + row * ntx + col), v[L]);
       }
     }
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const T d0 = v[1][c] - v[0][c], d1 = v[3][c] - v[2][c];
-      const T e0 = v[2][c] - v[0][c], e1 = v[3][c] - v[1][c];
-      f.V[c] = v[0][c];
-      f.X[c] = d0 + d1;
-      f.Y[c] = e0 + e1;
-      f.XY[c] = d1 - d0;
-      f.R[c] = f.X[c] + T(2) * e0;
-    }
-    if (use_d) {
-      T a0, a1, b0, b1;
-      ip2(T(1) - v[0][3], T(1) - v[1][3], a.k.c1, a.k.c2, a0, a1);
-      ip2(T(1) - v[2][3], T(1) - v[3][3], a.k.c1, a.k.c2, b0, b1);
-      ip2(a0, b0, a.k.c1, a.k.c2, f.o[0], f.o[2]);
-      ip2(a1, b1, a.k.c1, a.k.c2, f.o[1], f.o[3]);
-    }
+    elastic_face(v, f);
+    if (use_d) damage_face(v[0][3], v[1][3], v[2][3], v[3][3], a.k, f);
   };
   // TMA: thread 0 issues the copies of node layer kn into buffer b
   auto tma_issue = [&](int i0, int j0, int kn, int b) {
@@ -477,53 +446,12 @@ __device__ __forceinline__ void tile_body(const TileArgs<T>& a, const VoxMat<T>&
         if (eo >= 0 && gk >= 0) {
           const size_t e = plane_e * gk + eo;
           const bool own = own_xy && kk >= 1;
-          const TileK<T>& k = a.k;
-          // z modes of the element: sums (X, Y, XY) and differences (Mz, Xz, Yz, XYz) of the two faces
-          T X[3], Y[3], XY[3], Mz[3], Xz[3], Yz[3], XYz[3];
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            X[c] = fl.X[c] + fu.X[c];
-            Y[c] = fl.Y[c] + fu.Y[c];
-            XY[c] = fl.XY[c] + fu.XY[c];
-            Mz[c] = T(4) * (fu.V[c] - fl.V[c]) + (fu.R[c] - fl.R[c]);
-            Xz[c] = fu.X[c] - fl.X[c];
-            Yz[c] = fu.Y[c] - fl.Y[c];
-            XYz[c] = fu.XY[c] - fl.XY[c];
-          }
-          // d u_c / dz at [qy][qx]; the macro strain enters each strain component once, in the gradient
-          // term that component starts from
-          T Dz[3][2][2], Pz[3][2][2];
-#pragma unroll
-          for (int c = 0; c < 3; ++c)
-#pragma unroll
-            for (int qx = 0; qx < 2; ++qx) {
-              const T sx = qx ? k.g : -k.g;
-              const T A = Mz[c] + sx * Xz[c], B = Yz[c] + sx * XYz[c];
-              const T t = k.az * A + (EROWS ? (c == 0 ? E6[4] : (c == 1 ? E6[3] : E6[2])) : T(0));
-              Dz[c][0][qx] = t - k.bz * B;
-              Dz[c][1][qx] = t + k.bz * B;
-            }
           // coefficients of the material: lam and mu times the quadrature weight
           const T lw = COEF == kCoefIso ? m.lam[sl] * w : T(0), mw = COEF == kCoefIso ? m.mu[sl] * w : T(0);
           const T kap = T(m.kappa), okap = T(1) - kap;
-          // sums over the Gauss points of each half (qz = 0, 1) for the transposed gradient
-          T Sx[3][2], Sy[3][2], Sxy[3][2];
-#pragma unroll
-          for (int qz = 0; qz < 2; ++qz) {
-            const T sz = qz ? k.g : -k.g;
-            T Dx[3][2], Dy[3][2];  // [qy], [qx]
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-              const T Ax = X[c] + sz * Xz[c], Ay = Y[c] + sz * Yz[c], B = XY[c] + sz * XYz[c];
-              const T tx = k.ax * Ax + (EROWS && c == 0 ? E6[0] : T(0));
-              const T ty = k.ay * Ay + (EROWS && c == 0 ? E6[5] : (EROWS && c == 1 ? E6[1] : T(0)));
-              Dx[c][0] = tx - k.bx * B;
-              Dx[c][1] = tx + k.bx * B;
-              Dy[c][0] = ty - k.by * B;
-              Dy[c][1] = ty + k.by * B;
-            }
-            // degradation (and, on coarse levels, the moduli) of the half's four Gauss points
-            T gv[4], lm[8];
+          // degradation (and, on coarse levels, the moduli) of a half's four Gauss points
+          T gv[4], lm[8];
+          auto half = [&](int qz) {
             if (SLOT) {
               if (a.gq) {
 #pragma unroll
@@ -531,7 +459,7 @@ __device__ __forceinline__ void tile_body(const TileArgs<T>& a, const VoxMat<T>&
               } else if (d) {
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                  const T o = qz ? k.c2 * fl.o[q] + k.c1 * fu.o[q] : k.c1 * fl.o[q] + k.c2 * fu.o[q];
+                  const T o = intact_at(fl, fu, a.k, qz, q);
                   gv[q] = okap * (o * o) + kap;
                 }
               } else {
@@ -557,104 +485,41 @@ __device__ __forceinline__ void tile_body(const TileArgs<T>& a, const VoxMat<T>&
                 lm[4 + q] = __ldg(a.mu_q + 8 * e + 4 * qz + q);
               }
             }
-            T Px[3][2], Py[3][2];
+          };
+          auto stress = [&](int q, const T(&ep)[6], T(&sg)[6]) {
+            if constexpr (COEF == kCoefAniso) {
+              voigt_stress(m, sl, ep, sg);
+              const T gw = gv[q] * w;
 #pragma unroll
-            for (int qy = 0; qy < 2; ++qy)
-#pragma unroll
-              for (int qx = 0; qx < 2; ++qx) {
-                const int q = qx + 2 * qy;
-                T ep[6], sg[6];
-                ep[0] = Dx[0][qy];
-                ep[1] = Dy[1][qx];
-                ep[2] = Dz[2][qy][qx];
-                ep[3] = Dz[1][qy][qx] + Dy[2][qx];
-                ep[4] = Dz[0][qy][qx] + Dx[2][qy];
-                ep[5] = Dy[0][qx] + Dx[1][qy];
-                if constexpr (COEF == kCoefAniso) {
-                  voigt_stress(m, sl, ep, sg);
-                  const T gw = gv[q] * w;
-#pragma unroll
-                  for (int i = 0; i < 6; ++i) sg[i] *= gw;
-                } else {
-                  const T lg = COEF == kCoefIso ? lw * gv[q] : lm[q] * w;
-                  const T mg = COEF == kCoefIso ? mw * gv[q] : lm[4 + q] * w;
-                  const T mg2 = mg + mg;
-                  const T lt = lg * (ep[0] + ep[1] + ep[2]);
-                  sg[0] = mg2 * ep[0] + lt;
-                  sg[1] = mg2 * ep[1] + lt;
-                  sg[2] = mg2 * ep[2] + lt;
-                  sg[3] = mg * ep[3];
-                  sg[4] = mg * ep[4];
-                  sg[5] = mg * ep[5];
-                }
-                if (ENERGY && own) {
-#pragma unroll
-                  for (int i = 0; i < 6; ++i) tacc[kOutEnergy] += T(0.5) * sg[i] * ep[i];
-                }
-                // first contribution to a sum assigns, the others add
-                Px[0][qy] = qx == 0 ? sg[0] : Px[0][qy] + sg[0];
-                Px[1][qy] = qx == 0 ? sg[5] : Px[1][qy] + sg[5];
-                Px[2][qy] = qx == 0 ? sg[4] : Px[2][qy] + sg[4];
-                Py[0][qx] = qy == 0 ? sg[5] : Py[0][qx] + sg[5];
-                Py[1][qx] = qy == 0 ? sg[1] : Py[1][qx] + sg[1];
-                Py[2][qx] = qy == 0 ? sg[3] : Py[2][qx] + sg[3];
-                Pz[0][qy][qx] = qz == 0 ? sg[4] : Pz[0][qy][qx] + sg[4];
-                Pz[1][qy][qx] = qz == 0 ? sg[3] : Pz[1][qy][qx] + sg[3];
-                Pz[2][qy][qx] = qz == 0 ? sg[2] : Pz[2][qy][qx] + sg[2];
-              }
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-              Sx[c][qz] = Px[c][0] + Px[c][1];
-              Sy[c][qz] = Py[c][0] + Py[c][1];
-              Sxy[c][qz] = k.ax * (Px[c][1] - Px[c][0]) + k.ay * (Py[c][1] - Py[c][0]);
+              for (int i = 0; i < 6; ++i) sg[i] *= gw;
+            } else {
+              iso_stress(COEF == kCoefIso ? lw * gv[q] : lm[q] * w, COEF == kCoefIso ? mw * gv[q] : lm[4 + q] * w, ep,
+                         sg);
             }
-          }
-          // transposed gradient: the element's modal forces, split into its two faces
+            if (ENERGY && own) {
 #pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            const T p0 = Pz[c][0][0] + Pz[c][0][1], p1 = Pz[c][1][0] + Pz[c][1][1];
-            const T m0 = Pz[c][0][1] - Pz[c][0][0], m1 = Pz[c][1][1] - Pz[c][1][0];
-            const T T0 = p0 + p1, TY = p1 - p0, TX = m0 + m1, TXY = m1 - m0;
-            const T sx = Sx[c][0] + Sx[c][1], sy = Sy[c][0] + Sy[c][1];
+              for (int i = 0; i < 6; ++i) tacc[kOutEnergy] += T(0.5) * sg[i] * ep[i];
+            }
+          };
+          auto rows = [&](int c, T sx, T sy, T sz) {
             if (EROWS && own && e_live) {
               if (c == 0) {
                 tacc[0] += sx;
                 tacc[5] += sy;
-                tacc[4] += T0;
+                tacc[4] += sz;
               } else if (c == 1) {
                 tacc[1] += sy;
-                tacc[3] += T0;
+                tacc[3] += sz;
               } else {
-                tacc[2] += T0;
+                tacc[2] += sz;
               }
             }
-            const T fX = k.ax * sx, fY = k.ay * sy, fXY = k.g * (Sxy[c][0] + Sxy[c][1]);
-            const T fM = k.az * T0;
-            const T fXz = k.bx * (Sx[c][1] - Sx[c][0]) + k.bz * TX;
-            const T fYz = k.by * (Sy[c][1] - Sy[c][0]) + k.bz * TY;
-            const T fXYz = k.g * (k.g * (Sxy[c][1] - Sxy[c][0]) + k.bz * TXY);
-            lo.M[c] -= fM;
-            lo.X[c] += fX - fXz;
-            lo.Y[c] += fY - fYz;
-            lo.XY[c] += fXY - fXYz;
-            pend.M[c] = fM;
-            pend.X[c] = fX + fXz;
-            pend.Y[c] = fY + fYz;
-            pend.XY[c] = fXY + fXYz;
-          }
+          };
+          elastic_element<EROWS>(fl, fu, a.k, E6, half, stress, rows, lo, pend);
         }
         fl = fu;
         if (kk >= 1) {
-          // corner forces on node layer ke: corner L = (x side, y side), component c at FC[(3 L + c) exy + tid]
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            const T mm = lo.M[c] - lo.Y[c], mp = lo.M[c] + lo.Y[c];
-            const T xm = lo.X[c] - lo.XY[c], xp = lo.X[c] + lo.XY[c];
-            FC[c * exy + tid] = mm - xm;
-            FC[(3 + c) * exy + tid] = mm + xm;
-            FC[(6 + c) * exy + tid] = mp - xp;
-            FC[(9 + c) * exy + tid] = mp + xp;
-          }
+          corner_forces(lo, FC, exy, tid);  // of node layer ke
         }
       }
       if (kk == 0) continue;  // the first element layer only fills pend
@@ -668,7 +533,7 @@ __device__ __forceinline__ void tile_body(const TileArgs<T>& a, const VoxMat<T>&
           const size_t n = plane_n * ke + no;
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
-            T v = (FC[c * exy + e11] + FC[(3 + c) * exy + e01]) + (FC[(6 + c) * exy + e10] + FC[(9 + c) * exy + e00]);
+            T v = node_force(FC, exy, c, e11, e01, e10, e00);
             if (mk_cur & (1 << c)) v = T(0);
             const size_t i = 3 * n + c;
             const T xin = nval(ib0, c, nj + 1, ni + 1);

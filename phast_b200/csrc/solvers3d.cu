@@ -385,7 +385,13 @@ static int mech_solve_impl(const phastb_voxel_grid* g, const phastb_voxel_materi
                   closure ? nullptr : h8_apply_dot_slot(v, 8, scratch)};
   PcgResult pr{};
   if ((st = cuda_status(cudaMemcpyAsync(xw, x_out, sizeof(double) * n, cudaMemcpyDeviceToDevice, s)))) return st;
-  if ((st = pcg_run<double>(A, n, w, bf, invd, nullptr, xw, thr, maxiter, check_every, PCG_FREEZE, 0.0, &pr, s)))
+  // small cells: all iterations in one launch, with the element scratch as its exchange words
+  const PcgLoop loop = [&](int mi) {
+    return h8_mech_brick_pcg(v, mm, slot, gq, d, fixed, w, scratch, align_up(24 * sizeof(double) * (size_t)v.n_elem),
+                             xw, invd, mi, PCG_FREEZE, s);
+  };
+  if ((st = pcg_run<double>(A, n, w, bf, invd, nullptr, xw, thr, maxiter, check_every, PCG_FREEZE, 0.0, &pr, s,
+                            closure ? nullptr : &loop)))
     return st;
   { note_launch(); where_kernel<<<G, kThreads, 0, s>>>(n, fixed, xw, xc, x_out); }
   if ((st = last_launch_status())) return st;
