@@ -1,0 +1,43 @@
+"""The V-cycle with one smoothing step, whose residual, smoothing and sums are epilogues of the action (needs a B200).
+
+Level grids that do not fill a brick, free faces, a free macro strain, two and three levels, FP64 and
+mixed precision: each solve must end at the solution of the system that the elastic action defines.
+Tolerance: the stopping test is rtol ||b|| on the FP64 residual (mixed) or on a recursive residual that
+drifts from it by rounding only; a factor of two above it.
+"""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+CELLS = [((8, 8, 8), (True, True, True)), ((20, 12, 8), (False, True, True)), ((36, 28, 16), (True, True, True)),
+         ((16, 60, 24), (True, True, False))]
+RTOL = 1e-8
+
+
+@pytest.mark.parametrize("shape,periodic", CELLS)
+@pytest.mark.parametrize("mixed", [True, False])
+@pytest.mark.parametrize("levels,free_strain", [(3, False), (2, True)])
+def test_one_step_cycle(shape, periodic, mixed, levels, free_strain):
+    from phast_b200 import solid3d as s3
+    rng = np.random.default_rng(17)
+    h = (1.0 / shape[0], 1.1 / shape[0], 0.9 / shape[0])
+    slot = rng.integers(0, 2, int(np.prod(shape)))
+    phases = [s3.PhaseMaterial("mi_matrix", "isotropic", 0.5, "spectral", 3000.0, 0.35),
+              s3.PhaseMaterial("fibre", "isotropic", 0.2, "spectral", 9000.0, 0.3)]
+    load = (s3.LoadCase("zz", 2, (0.01,), (0, 1), (3, 4, 5)) if free_strain
+            else s3.LoadCase("zz", 2, (0.01,), (), (0, 1, 3, 4, 5)))
+    op = s3.PeriodicVoxelPhaseFieldOperator.from_slots(s3.VoxelGrid(shape, h, periodic=periodic), slot, phases,
+                                                       2 * h[0], 1e-6, load, pinned_node=0)
+    d = torch.as_tensor(rng.uniform(0.0, 0.6, op.n_red), device="cuda")
+    mask = op.mech_fixed_mask()
+    if not all(periodic):  # no rigid rotations of a cell with free faces: hold a random tenth of the nodes
+        held = torch.as_tensor(rng.random(op.n_red) < 0.1, device="cuda")
+        mask[:3 * op.n_red] |= held.repeat_interleave(3)
+    values = torch.where(mask, torch.as_tensor(rng.uniform(-1e-3, 1e-3, op.n_mech), device="cuda"), 0.0)
+    form = s3.MechForm("gmg", mixed=mixed, levels=levels, smooth_degree=1, coarse_degree=6)
+    x, info = s3.solve_constrained_form(op, form, fixed_mask=mask, fixed_values=values, d=d, rtol=RTOL, maxiter=2000)[:2]
+    act = op.mech_operator(d=d)
+    assert info.converged and bool((x[mask] == values[mask]).all())
+    assert float(act(x)[~mask].norm()) <= 2 * RTOL * float(act(values)[~mask].norm())
