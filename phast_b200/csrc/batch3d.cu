@@ -1104,6 +1104,29 @@ __global__ void __launch_bounds__(kThreads) bpcg_rz_kernel(BVec V, BPcg<T> w, in
   });
 }
 
+// bpcg_rz_kernel (not at the start) and bpcg_dir_kernel in one launch, with each cell's r . z from the
+// preconditioner (rz_red): see pcg_dir_rz_kernel.  A cell's first chunk stores its state.
+template <typename T>
+__global__ void __launch_bounds__(kThreads) bpcg_dir_rz_kernel(BVec V, BPcg<T> w, const char* rz_red) {
+  const BChunk ck = V.chunks[blockIdx.x];
+  const int c = ck.cell;
+  PcgState* S = w.st + c;
+  if (!S->active) return;
+  const double RZ = cell_out(rz_red, c)[0], old = S->rz_old;
+  const bool nonfinite = S->nonfinite || !isfinite(RZ);
+  const double beta = old > 0.0 ? RZ / old : 0.0;
+  if (!nonfinite) {
+    const T be = T(beta);
+    for (int i = ck.begin + threadIdx.x; i < ck.end; i += blockDim.x) w.p[i] = w.z[i] + be * w.p[i];
+  }
+  if (threadIdx.x == 0 && ck.j == 0) {
+    S->nonfinite = nonfinite;
+    S->beta = beta;
+    S->rz = RZ;
+    if (nonfinite) S->active = 0;
+  }
+}
+
 // alpha from the action's p.Ap; x += alpha p; r -= alpha Ap; rr and the convergence test
 template <typename T>
 __global__ void __launch_bounds__(kThreads) bpcg_update_pre_kernel(BVec V, BPcg<T> w, T* __restrict__ x,
@@ -1136,6 +1159,7 @@ __global__ void __launch_bounds__(kThreads) bpcg_update_pre_kernel(BVec V, BPcg<
       return;
     }
     st.alpha = alpha;
+    st.rz_old = st.rz;
     st.steps += 1;
     if (!isfinite(RR)) st.nonfinite = 1;
     st.rr = RR;
@@ -1523,6 +1547,10 @@ int bpcg_run_pre(const phastb_batch* B, const BatchOp<float>& A, const GraphKey&
       if ((e = A(w.p, w.Ap, guard, kStateInts, true, s))) return e;
       { note_launch(); bpcg_update_pre_kernel<float><<<V.n_chunks, kThreads, 0, s>>>(V, w, x, dot_red); }
       if ((e = bg_precond(M, w.r, w.z, s))) return e;
+      if (M.deg == 1) {  // (the one-step post-smoother leaves r . z per cell)
+        { note_launch(); bpcg_dir_rz_kernel<float><<<V.n_chunks, kThreads, 0, s>>>(V, w, M.L[0].red); }
+        continue;
+      }
       { note_launch(); bpcg_rz_kernel<float><<<V.n_chunks, kThreads, 0, s>>>(V, w, 0); }
       { note_launch(); bpcg_dir_kernel<float><<<V.n_chunks, kThreads, 0, s>>>(V, w); }
     }

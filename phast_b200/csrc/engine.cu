@@ -702,6 +702,7 @@ __global__ void __launch_bounds__(kThreads) pcg_update_kernel(int n, PcgWs<T> w,
         }
       } else {
         st.rr = RR;
+        st.rz_old = st.rz;
         if (!(RR > st.thr_sq)) {
           st.converged = 1;
           st.active = 0;
@@ -740,16 +741,41 @@ __global__ void __launch_bounds__(kThreads) pcg_update_dot_kernel(int n, PcgWs<T
   const T a = T(alpha);
   double rz = 0, rr = 0;
   if (ok) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const int t0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    // V values of a thread's pass in one access of each vector
+    constexpr int V = 16 / sizeof(T);
+    using Vec = typename Vec16<T>::type;
+    int tail = 0;
+    if (aligned16(x) && (!inv_diag || aligned16(inv_diag))) {
+      tail = n / V * V;
+      for (int c = t0; c < n / V; c += step) {
+        T xv[V], pv[V], rv[V], av[V], dv[V], zv[V];
+        *reinterpret_cast<Vec*>(xv) = reinterpret_cast<const Vec*>(x)[c];
+        *reinterpret_cast<Vec*>(pv) = reinterpret_cast<const Vec*>(w.p)[c];
+        *reinterpret_cast<Vec*>(rv) = reinterpret_cast<const Vec*>(w.r)[c];
+        *reinterpret_cast<Vec*>(av) = reinterpret_cast<const Vec*>(w.Ap)[c];
+        if (!custom_pre && inv_diag) *reinterpret_cast<Vec*>(dv) = reinterpret_cast<const Vec*>(inv_diag)[c];
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+          xv[k] = xv[k] + a * pv[k];
+          rv[k] = rv[k] - a * av[k];
+          rr += double(rv[k]) * double(rv[k]);
+          zv[k] = !custom_pre && inv_diag ? rv[k] * dv[k] : rv[k];
+          rz += double(rv[k]) * double(zv[k]);
+        }
+        reinterpret_cast<Vec*>(x)[c] = *reinterpret_cast<const Vec*>(xv);
+        reinterpret_cast<Vec*>(w.r)[c] = *reinterpret_cast<const Vec*>(rv);
+        if (!custom_pre) reinterpret_cast<Vec*>(w.z)[c] = *reinterpret_cast<const Vec*>(zv);
+      }
+    }
+    for (int i = tail + t0; i < n; i += step) {
       x[i] = x[i] + a * w.p[i];
       const T r = w.r[i] - a * w.Ap[i];
       w.r[i] = r;
       rr += double(r) * double(r);
-      if (!custom_pre) {
-        const T z = inv_diag ? r * inv_diag[i] : r;
-        w.z[i] = z;
-        rz += double(r) * double(z);
-      }
+      const T z = !custom_pre && inv_diag ? r * inv_diag[i] : r;
+      if (!custom_pre) w.z[i] = z;
+      rz += double(r) * double(z);
     }
   }
   double v2[2] = {rz, rr};
@@ -775,6 +801,7 @@ __global__ void __launch_bounds__(kThreads) pcg_update_dot_kernel(int n, PcgWs<T
         st.active = 0;
       } else {
         st.alpha = alpha;
+        st.rz_old = st.rz;
         if (mode != PCG_PERIODIC) st.steps += 1;
         if (!isfinite(RR) || (!custom_pre && !isfinite(RZ))) st.nonfinite = 1;
         if (mode == PCG_PERIODIC) {
@@ -816,12 +843,14 @@ __global__ void pcg_dir_kernel(int n, PcgWs<T> w) {
 }
 
 // pcg_rz_kernel (not at the start) and pcg_dir_kernel in one launch, with r . z from the preconditioner: every
-// block derives beta from the same scalars, and the last one to finish stores the state.
+// block derives beta from the same scalars (rz_old is not written here), so one block stores the state at once;
+// waiting for the last block to arrive instead cost two of the kernel's five us on 64^3.  A block that starts after
+// a breakdown was stored leaves p as it is; nothing reads p then.
 template <typename T>
 __global__ void __launch_bounds__(kThreads) pcg_dir_rz_kernel(int n, PcgWs<T> w, const double* __restrict__ rz_in,
                                                               int mode) {
   if (!w.st->active) return;
-  const double RZ = *rz_in, old = w.st->rz;
+  const double RZ = *rz_in, old = w.st->rz_old;
   const bool nonfinite = w.st->nonfinite || !isfinite(RZ);
   const bool breakdown = w.st->breakdown || (mode == PCG_STRICT && !(RZ > 0.0));
   const double beta = (mode == PCG_STRICT) ? RZ / old : ((old > 0.0) ? RZ / old : 0.0);
@@ -830,14 +859,13 @@ __global__ void __launch_bounds__(kThreads) pcg_dir_rz_kernel(int n, PcgWs<T> w,
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
       w.p[i] = w.z[i] + be * w.p[i];
   }
-  if (arrive_last(w.counter) && threadIdx.x == 0) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
     PcgState& st = *w.st;
     st.nonfinite = nonfinite;
     st.breakdown = breakdown;
     st.beta = beta;
     st.rz = RZ;
     if (nonfinite || breakdown) st.active = 0;
-    *w.counter = 0u;
   }
 }
 
@@ -896,7 +924,7 @@ int pcg_run_thr(const LinOp<T>& A, int n, const PcgWs<T>& w, const T* b, const T
     for (int k = 0; k < k_iters; ++k) {
       if (A.apply_dot) {
         if ((e = A.apply_dot(A.ctx, w.p, w.Ap, active, s))) return e;
-        { note_launch(); pcg_update_dot_kernel<T><<<G, kThreads, 0, s>>>(n, w, x, inv_diag, custom, mode, check_every, A.dot_out); }
+        { note_launch(); pcg_update_dot_kernel<T><<<std::min(G, kReduceBlocks), kThreads, 0, s>>>(n, w, x, inv_diag, custom, mode, check_every, A.dot_out); }
       } else {
         if ((e = A(w.p, w.Ap, active, s))) return e;
         { note_launch(); pcg_alpha_kernel<T><<<G, kThreads, 0, s>>>(n, w, mode); }

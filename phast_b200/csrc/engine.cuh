@@ -72,6 +72,7 @@ enum PcgMode { PCG_FREEZE = 0, PCG_STRICT = 1, PCG_PERIODIC = 2 };
 
 struct PcgState {
   double rz, rr, rr0, thr_sq, alpha, beta;
+  double rz_old;    // rz of the iteration before, set with alpha for a preconditioner that forms r . z itself
   int active;       // iterating (guard for the operator)
   int breakdown, nonfinite;
   int steps;        // iterations that moved the iterate

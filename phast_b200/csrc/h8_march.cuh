@@ -47,22 +47,10 @@ __device__ __forceinline__ void cp_async_word_or_zero(T* smem, const T* gmem, bo
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(s), "l"(gmem), "n"(sizeof(T)), "r"(n)
                : "memory");
 }
-__device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // Staged per-element arrays live chunk-major in shared memory: chunk c (16
 // bytes) of the element owned by thread t sits at base + (c * n + t) * 16, so a
 // warp reading one chunk touches consecutive 16-byte units (no bank conflicts).
-template <typename T>
-struct Vec16;
-template <>
-struct Vec16<float> {
-  using type = float4;
-};
-template <>
-struct Vec16<double> {
-  using type = double2;
-};
-
 // Copies n_chunks 16-byte chunks of src into chunks c0.. of thread t's column.
 __device__ __forceinline__ void stage_chunks(unsigned char* base, int n, int t, int c0, const void* src,
                                              int n_chunks) {
