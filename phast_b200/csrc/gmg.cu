@@ -21,6 +21,7 @@
 // * On the fine level the pinned node and the macro-strain rows are held at
 //   zero by the mask; the macro-strain rows of the preconditioned vector are a
 //   Jacobi step (diagonal of the E block).
+#include "h8_cheb.cuh"
 #include "engine.cuh"
 #include "h8_kernels.cuh"
 #include "h8_tile.cuh"
@@ -516,6 +517,7 @@ struct Gmg {
   int deg, deg_coarse;
   double safety;         // Chebyshev interval [lmax/30, safety * lmax]
   const int* guard;      // set per preconditioner call: the Krylov engine's "still iterating" flag
+  void* exchange;        // FP32: words of the coarsest level's one-launch solve (h8_cheb.cu)
 };
 
 template <typename T>
@@ -637,6 +639,24 @@ static int chebyshev(const Gmg<T>& M, int l, int deg, bool from_zero, bool need_
   const double theta = 0.5 * (bmax + amin), delta = 0.5 * (bmax - amin), sigma = theta / delta;
   // one step from zero: the residual is b - A x, without the recurrence's vectors
   const bool one = from_zero && deg == 1;
+  if constexpr (sizeof(T) == 4) {
+    // the coarsest level's solve: every step in one launch where the level is small enough
+    if (l > 0 && l == M.nlev - 1 && from_zero && !need_res && deg > 1 && deg - 1 <= kChebMaxSteps) {
+      double c1[kChebMaxSteps], c2[kChebMaxSteps], ro = 1.0 / sigma;
+      for (int k = 1; k < deg; ++k) {
+        const double rho = 1.0 / (2.0 * sigma - ro);
+        c1[k - 1] = rho * ro;
+        c2[k - 1] = 2.0 * rho / delta;
+        ro = rho;
+      }
+      st = coarse_cheb_launch(L.g, L.lam, L.mu, L.b, L.invd, L.x, bsums, 1.0 / theta, c1, c2, deg - 1,
+                              summed ? &M.rw : nullptr, M.exchange, M.guard, s);
+      if (st != PHASTB_UNSUPPORTED) {
+        if (summed) *summed = true;
+        return st;
+      }
+    }
+  }
   if (from_zero) {
     { note_launch(); gmg_cheb_first_b<T><<<G, kThreads, 0, s>>>(n, L.b, L.invd, T(1.0 / theta), one ? nullptr : L.res, L.dvec, L.x, bsums, M.guard); }
     if (one) return need_res ? level_residual(M, l, L.x, L.res, false, 0.0, s) : last_launch_status();
@@ -748,6 +768,12 @@ __global__ void gmg_fine_mask(int n_mech, int nu, const uint8_t* __restrict__ fi
 
 // Bytes of one GMG hierarchy in precision T for a fine grid f (levels >= 2).
 template <typename T>
+static VoxGeom gmg_coarsest(VoxGeom g, int levels) {
+  for (int l = 1; l < levels; ++l) g = coarse_geom<T>(g);
+  return g;
+}
+
+template <typename T>
 size_t gmg_hier_bytes(const VoxGeom& f, int levels) {
   size_t tot = 0;
   VoxGeom g = f;
@@ -760,6 +786,7 @@ size_t gmg_hier_bytes(const VoxGeom& f, int levels) {
   tot += align_up(3 * (size_t)f.n_red + 6);  // fine mask
   tot += h8_scratch_bytes(f, sizeof(T) == 4 ? PHASTB_F32 : PHASTB_F64);
   tot += red_ws_bytes();
+  if (sizeof(T) == 4) tot += coarse_cheb_bytes(gmg_coarsest<T>(f, levels));
   return tot;
 }
 
@@ -795,6 +822,8 @@ static char* gmg_carve(Gmg<T>& M, const VoxGeom& f, int levels, char* p) {
   p += h8_scratch_bytes(f, sizeof(T) == 4 ? PHASTB_F32 : PHASTB_F64);
   M.rw = red_ws(p);
   p += red_ws_bytes();
+  M.exchange = p;
+  if (sizeof(T) == 4) p += coarse_cheb_bytes(gmg_coarsest<T>(f, levels));
   return p;
 }
 
@@ -816,6 +845,7 @@ static int gmg_setup(Gmg<T>& M, const VoxMat<T>& mat, const uint8_t* slot, const
   const VoxGeom& f = M.lv[0].g;
   const int nu = 3 * f.n_red, nm = nu + 6;
   if ((st = cuda_status(cudaMemsetAsync(M.rw.counter, 0, sizeof(unsigned), s)))) return st;
+  if (sizeof(T) == 4 && (st = coarse_cheb_reset(M.lv[M.nlev - 1].g, M.exchange, s))) return st;
   { note_launch(); gmg_fine_mask<<<grid_for(nm), kThreads, 0, s>>>(nm, nu, fixed, const_cast<uint8_t*>(M.mask)); }
   // fine diagonal (its E rows serve the Jacobi step of the E block)
   RedWs sw = red_ws(static_cast<char*>(M.scratch) + (h8_scratch_bytes(f, sizeof(T) == 4 ? PHASTB_F32 : PHASTB_F64) -

@@ -61,6 +61,11 @@ __device__ __forceinline__ bool wait_tagged(const Tagged* p, unsigned long long 
   return true;
 }
 
+// Barrier of the `threads` threads that share id (1..15) inside a block.
+__device__ __forceinline__ void sub_barrier(int id, int threads) {
+  asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
+}
+
 constexpr int kGridValues = 3;     // values of one reduction
 constexpr int kGridBlocks = 148;   // at most one block per SM
 constexpr int kGridDirect = 32;    // up to so many blocks read one another's words directly

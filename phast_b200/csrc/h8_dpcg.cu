@@ -79,10 +79,6 @@ struct BrickLayout {
   }
 };
 
-__device__ __forceinline__ void sub_barrier(int id, int threads) {
-  asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
-}
-
 template <typename T, int OX, int OY, int NS>
 __global__ void __launch_bounds__(kT, 1) h8_dpcg_kernel(BrickArgs<T> a) {
   using L = BrickLayout<T, OX, OY, NS>;

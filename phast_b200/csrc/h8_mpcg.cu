@@ -69,10 +69,6 @@ struct MBrickLayout {
   }
 };
 
-__device__ __forceinline__ void sub_barrier(int id, int threads) {
-  asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
-}
-
 template <int COEF, int OX, int OY>
 __global__ void __launch_bounds__(kT, 1) h8_mpcg_kernel(MBrickArgs a, VoxMat<T> m) {
   using L = MBrickLayout<OX, OY>;

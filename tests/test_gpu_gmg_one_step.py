@@ -1,6 +1,6 @@
 """The V-cycle with one smoothing step, whose residual, smoothing and sums are epilogues of the action (needs a B200).
 
-Level grids that do not fill a brick, free faces, a free macro strain, two and three levels, FP64 and
+Level grids that do not fill a brick or split into sub-bricks (the coarsest level's one-launch solve), free faces, a free macro strain, two and three levels, FP64 and
 mixed precision: each solve must end at the solution of the system that the elastic action defines.
 Tolerance: the stopping test is rtol ||b|| on the FP64 residual (mixed) or on a recursive residual that
 drifts from it by rounding only; a factor of two above it.
@@ -12,7 +12,8 @@ import torch
 pytestmark = pytest.mark.gpu
 
 CELLS = [((8, 8, 8), (True, True, True)), ((20, 12, 8), (False, True, True)), ((36, 28, 16), (True, True, True)),
-         ((16, 60, 24), (True, True, False))]
+         ((16, 60, 24), (True, True, False)), ((48, 44, 48), (True, True, True)), ((64, 64, 60), (True, False, True)),
+         ((80, 72, 80), (True, True, True))]
 RTOL = 1e-8
 
 
