@@ -16,6 +16,7 @@
 //   FP32 inner solves under FP64 iterative refinement (mixed_precision_cg.py);
 //   primal active-set box-KKT damage with a Dirichlet PCG per set
 //   (solvers/box_kkt_h8.py:256-778).
+#include "h8_cheb.cuh"
 #include "engine.cuh"
 #include "h8_kernels.cuh"
 #include "h8_tile.cuh"
@@ -1263,6 +1264,7 @@ struct BGmg {
   int deg, deg_coarse;
   const int* guard;      // the Krylov engine's per-cell active flags
   int gstride;
+  void* exchange;        // words of the coarsest level's one-launch solve (h8_cheb.cu)
 };
 
 size_t bgmg_bytes(const phastb_batch* B) {
@@ -1279,6 +1281,7 @@ size_t bgmg_bytes(const phastb_batch* B) {
     cv.take<char>(n_red_ws(P));
   }
   cv.take<uint8_t>((size_t)B->n_mech);
+  cv.take<char>(coarse_cheb_bytes(B->nlev > 1 ? B->lev[B->nlev - 2]->n_nodes : 0));
   return cv.used;
 }
 
@@ -1302,6 +1305,7 @@ void bgmg_carve(BGmg& M, const phastb_batch* B, char* base) {
     L.ared = cv.take<char>(n_red_ws(L.P));
   }
   M.mask = cv.take<uint8_t>((size_t)B->n_mech);
+  M.exchange = cv.take<char>(coarse_cheb_bytes(B->nlev > 1 ? B->lev[B->nlev - 2]->n_nodes : 0));
 }
 
 TileBatchArgs<float> bg_args(const BGmg& M, int l, const float* x) {
@@ -1378,6 +1382,23 @@ int bg_chebyshev(const BGmg& M, int l, int deg, bool from_zero, bool need_res, c
   const double a = 1.0 / 30.0, bm = M.safety;  // interval [lmax/30, safety lmax] relative to lmax
   const double sigma = (bm + a) / (bm - a);
   const bool one = from_zero && deg == 1;
+  // the coarsest level's solve: every step of every cell in one launch where they fit
+  if (summed && l > 0 && from_zero && !need_res && deg > 1 && deg - 1 <= kChebMaxSteps) {
+    double c1[kChebMaxSteps], c2[kChebMaxSteps], ro = 1.0 / sigma;
+    for (int k = 1; k < deg; ++k) {
+      const double rho = 1.0 / (2.0 * sigma - ro);
+      c1[k - 1] = rho * ro;
+      c2[k - 1] = 2.0 * rho;
+      ro = rho;
+    }
+    st = coarse_cheb_batch_launch(L.P->d_cells, L.P->cells.data(), L.P->n_cells, L.P->n_nodes, L.lam, L.mu, L.b,
+                                  L.invd, L.x, bsum_red, L.inv_theta, L.inv_delta, c1, c2, deg - 1, L.red, M.exchange,
+                                  M.guard, M.gstride, s);
+    if (st != PHASTB_UNSUPPORTED) {
+      *summed = true;
+      return st;
+    }
+  }
   if (from_zero) {
     { note_launch(); bg_first_b_kernel<<<V.n_chunks, kThreads, 0, s>>>(V, L.P->d_cells, L.b, L.invd, L.inv_theta, one ? nullptr : L.res, L.dvec, L.x, bsum_red, M.guard, M.gstride); }
     if (one) return need_res ? bg_level_residual(M, l, L.x, L.res, false, s) : last_launch_status();
@@ -1462,6 +1483,7 @@ int bg_setup(BGmg& M, const phastb_batch* B, char* scratch, int power_iters, boo
   int st;
   M.guard = nullptr;
   M.gstride = 0;
+  if (M.nlev > 1 && (st = coarse_cheb_reset(M.L[M.nlev - 1].P->n_nodes, M.exchange, s))) return st;
   for (int l = 0; l < M.nlev; ++l) {
     const BLevel& L = M.L[l];
     float* v[7] = {L.diag, L.invd, L.x, L.b, L.res, L.dvec, L.Ad};

@@ -786,7 +786,7 @@ size_t gmg_hier_bytes(const VoxGeom& f, int levels) {
   tot += align_up(3 * (size_t)f.n_red + 6);  // fine mask
   tot += h8_scratch_bytes(f, sizeof(T) == 4 ? PHASTB_F32 : PHASTB_F64);
   tot += red_ws_bytes();
-  if (sizeof(T) == 4) tot += coarse_cheb_bytes(gmg_coarsest<T>(f, levels));
+  if (sizeof(T) == 4) tot += coarse_cheb_bytes(gmg_coarsest<T>(f, levels).n_red);
   return tot;
 }
 
@@ -823,7 +823,7 @@ static char* gmg_carve(Gmg<T>& M, const VoxGeom& f, int levels, char* p) {
   M.rw = red_ws(p);
   p += red_ws_bytes();
   M.exchange = p;
-  if (sizeof(T) == 4) p += coarse_cheb_bytes(gmg_coarsest<T>(f, levels));
+  if (sizeof(T) == 4) p += coarse_cheb_bytes(gmg_coarsest<T>(f, levels).n_red);
   return p;
 }
 
@@ -845,7 +845,7 @@ static int gmg_setup(Gmg<T>& M, const VoxMat<T>& mat, const uint8_t* slot, const
   const VoxGeom& f = M.lv[0].g;
   const int nu = 3 * f.n_red, nm = nu + 6;
   if ((st = cuda_status(cudaMemsetAsync(M.rw.counter, 0, sizeof(unsigned), s)))) return st;
-  if (sizeof(T) == 4 && (st = coarse_cheb_reset(M.lv[M.nlev - 1].g, M.exchange, s))) return st;
+  if (sizeof(T) == 4 && (st = coarse_cheb_reset(M.lv[M.nlev - 1].g.n_red, M.exchange, s))) return st;
   { note_launch(); gmg_fine_mask<<<grid_for(nm), kThreads, 0, s>>>(nm, nu, fixed, const_cast<uint8_t*>(M.mask)); }
   // fine diagonal (its E rows serve the Jacobi step of the E block)
   RedWs sw = red_ws(static_cast<char*>(M.scratch) + (h8_scratch_bytes(f, sizeof(T) == 4 ? PHASTB_F32 : PHASTB_F64) -

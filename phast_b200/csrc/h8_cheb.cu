@@ -33,7 +33,25 @@ struct ChebArgs {
   T* x;
   const double* bsums;
   RedWs ws;       // component sums of x at ws.out (counter null: none)
-  Tagged* words;  // [2][n_red]
+  Tagged* words;  // one per node, and again word_stride further on
+  long long word_stride;
+  unsigned *epoch, *err;  // epoch: one word per block of the launch
+  const int* guard;
+};
+
+// Several cells of a packed batch (BatchCell): the arrays hold the cells' vectors one after another, factors and
+// reductions are per cell.
+struct ChebBatchArgs {
+  const BatchCell* cells;
+  int n_cells, kz, steps, guard_stride;
+  double c1[kChebMaxSteps], c2[kChebMaxSteps];  // c2: in units of inv_delta
+  const double *inv_theta, *inv_delta;
+  const T *lam, *mu, *b, *invd;
+  T* x;
+  const char* bsums;  // per-cell workspaces (sums of b in, sums of x out)
+  char* sums;
+  Tagged* words;
+  long long word_stride;
   unsigned *epoch, *err;
   const int* guard;
 };
@@ -86,8 +104,9 @@ __device__ __forceinline__ bool wait_node(const Tagged* p, unsigned tag, T (&v)[
   return true;
 }
 
+// Brick vb of the vgrid bricks of one grid.
 template <int NS>
-__global__ void __launch_bounds__(NS* TPS, 1) h8_cheb_kernel(ChebArgs a) {
+__device__ __forceinline__ void cheb_body(const ChebArgs& a, int vb, int vgrid) {
   if (a.guard && *a.guard == 0) return;
   constexpr int kT = NS * TPS;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -102,7 +121,7 @@ __global__ void __launch_bounds__(NS* TPS, 1) h8_cheb_kernel(ChebArgs a) {
   T* Q = reinterpret_cast<T*>(smem + lay.q) + (size_t)sub * (kz + 1) * 16 * EXY;
   int *HN = reinterpret_cast<int*>(smem + lay.hn), *HB = reinterpret_cast<int*>(smem + lay.hb);
   __shared__ int s_halo, s_lost;
-  const int txy = blockIdx.x % a.tiles_xy, bz = blockIdx.x / a.tiles_xy;
+  const int txy = vb % a.tiles_xy, bz = vb / a.tiles_xy;
   const int i0 = (txy % a.tiles_x) * OX, j0 = (txy / a.tiles_x) * OY, k0 = bz * NS * kz;
   const int nk = min(NS * kz, g.rz - k0);                      // node layers of the block
   const int wx = min(OX, g.rx - i0), wy = min(OY, g.ry - j0);  // owned nodes per axis
@@ -188,7 +207,7 @@ __global__ void __launch_bounds__(NS* TPS, 1) h8_cheb_kernel(ChebArgs a) {
     const bool last = it + 1 == a.steps;
     const unsigned tag = epoch + 1u + (unsigned)it;
     // a word is written again two steps later, when its readers have sent what they formed from it
-    Tagged* words = a.words + (size_t)(it & 1) * g.n_red;
+    Tagged* words = a.words + (it & 1 ? a.word_stride : 0);
     const T c1 = a.c1[it], c2 = a.c2[it];
     if (K > 0) {
       Face<T> fl;
@@ -272,18 +291,97 @@ __global__ void __launch_bounds__(NS* TPS, 1) h8_cheb_kernel(ChebArgs a) {
     }
   }
   if (tid == 0) a.epoch[blockIdx.x] = epoch + (unsigned)a.steps;
-  if (a.ws.counter) reduce_multi<3>(acc, a.ws);
+  if (a.ws.counter) {
+    __shared__ double sh[32 * 3];
+    block_sum_multi<3>(acc, sh);
+    if (tid == 0) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) a.ws.part[c * kMaxPartials + vb] = acc[c];
+    }
+    if (arrive_last_n(a.ws.counter, vgrid)) {
+      double f[3];
+      fold_sum_multi<3>(a.ws.part, kMaxPartials, vgrid, f, sh);
+      if (tid == 0) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) a.ws.out[c] = f[c];
+        *a.ws.counter = 0u;
+      }
+    }
+  }
 }
 
 template <int NS>
-int launch(const ChebArgs& a0, int grid, cudaStream_t s) {
-  ChebArgs a = a0;
+__global__ void __launch_bounds__(NS* TPS, 1) h8_cheb_kernel(ChebArgs a) {
+  cheb_body<NS>(a, blockIdx.x, gridDim.x);
+}
+
+template <int NS>
+__host__ __device__ __forceinline__ int cheb_blocks(const VoxGeom& g, int kz) {
+  return ((g.rx + OX - 1) / OX) * ((g.ry + OY - 1) / OY) * ((g.rz + NS * kz - 1) / (NS * kz));
+}
+
+template <int NS>
+__global__ void __launch_bounds__(NS* TPS, 1) h8_cheb_batch_kernel(ChebBatchArgs b) {
+  __shared__ ChebArgs sa;
+  __shared__ int s_vb, s_vgrid;
+  if (threadIdx.x == 0) {
+    int c = 0, vb = blockIdx.x, n = cheb_blocks<NS>(b.cells[0].g, b.kz);
+    while (vb >= n) {  // (the grid is the sum over the cells)
+      vb -= n;
+      n = cheb_blocks<NS>(b.cells[++c].g, b.kz);
+    }
+    const BatchCell& cl = b.cells[c];
+    sa.g = cl.g;
+    sa.tiles_x = (cl.g.rx + OX - 1) / OX;
+    sa.tiles_xy = sa.tiles_x * ((cl.g.ry + OY - 1) / OY);
+    sa.kz = b.kz;
+    sa.steps = b.steps;
+    sa.k = cl.kf;
+    sa.inv_theta = T(b.inv_theta[c]);
+    for (int i = 0; i < b.steps; ++i) {
+      sa.c1[i] = T(b.c1[i]);
+      sa.c2[i] = T(b.c2[i] * b.inv_delta[c]);
+    }
+    sa.lam = b.lam + 8 * cl.elem_off;
+    sa.mu = b.mu + 8 * cl.elem_off;
+    sa.b = b.b + cl.mech_off;
+    sa.invd = b.invd + cl.mech_off;
+    sa.x = b.x + cl.mech_off;
+    sa.bsums = b.bsums ? red_ws(const_cast<char*>(b.bsums) + (size_t)c * red_ws_bytes()).out : nullptr;
+    sa.ws = red_ws(b.sums + (size_t)c * red_ws_bytes());
+    sa.words = b.words + cl.node_off;
+    sa.word_stride = b.word_stride;
+    sa.epoch = b.epoch;
+    sa.err = b.err;
+    sa.guard = b.guard ? b.guard + (size_t)c * b.guard_stride : nullptr;
+    s_vb = vb;
+    s_vgrid = n;
+  }
+  __syncthreads();
+  cheb_body<NS>(sa, s_vb, s_vgrid);
+}
+
+// Opt-in to the shared memory of every depth, and how many blocks of depth kz the device holds at once (0: none).
+template <int NS, class Kernel>
+int resident_blocks(Kernel kern, int kz) {
+  int dev = 0, sms = 0, coop = 0, per = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ChebLayout<NS>(kMaxDepth).total) !=
+          cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, NS * TPS, ChebLayout<NS>(kz).total) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return std::min(sms * per, kChebBlocks);
+}
+
+template <int NS, class Kernel, class Args>
+int launch(Kernel kern, Args a, int grid, cudaStream_t s) {
   void* args[] = {&a};
-  const size_t bytes = ChebLayout<NS>(a.kz).total;
-  if (cudaFuncSetAttribute(h8_cheb_kernel<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)ChebLayout<NS>(kMaxDepth).total) != cudaSuccess ||
-      cudaLaunchCooperativeKernel((const void*)h8_cheb_kernel<NS>, dim3(grid), dim3(NS * TPS), args, bytes, s) !=
-          cudaSuccess) {
+  if (cudaLaunchCooperativeKernel((const void*)kern, dim3(grid), dim3(NS * TPS), args, ChebLayout<NS>(a.kz).total, s) !=
+      cudaSuccess) {
     cudaGetLastError();
     return PHASTB_UNSUPPORTED;
   }
@@ -291,38 +389,43 @@ int launch(const ChebArgs& a0, int grid, cudaStream_t s) {
   return PHASTB_OK;
 }
 
-}  // namespace
-
-size_t coarse_cheb_bytes(const VoxGeom& g) {
-  return align_up(2 * sizeof(Tagged) * (size_t)g.n_red) + align_up(sizeof(unsigned) * (kGridBlocks + 1));
+// One grid with a block per SM at most: more SMs than that only lengthen the rim.
+template <int NS>
+int try_cell(ChebArgs& a, int kz, cudaStream_t s) {
+  const int grid = cheb_blocks<NS>(a.g, kz);
+  a.kz = kz;
+  if (grid > kGridBlocks || grid > resident_blocks<NS>(h8_cheb_kernel<NS>, kz)) return PHASTB_UNSUPPORTED;
+  return launch<NS>(h8_cheb_kernel<NS>, a, grid, s);
 }
 
-int coarse_cheb_reset(const VoxGeom& g, void* exchange, cudaStream_t s) {
-  return cuda_status(cudaMemsetAsync(exchange, 0, coarse_cheb_bytes(g), s));
+// All cells of a batch at once, several blocks per SM where they fit.
+template <int NS>
+int try_batch(ChebBatchArgs& a, const BatchCell* cells, int kz, cudaStream_t s) {
+  long long grid = 0;
+  for (int c = 0; c < a.n_cells; ++c) grid += cheb_blocks<NS>(cells[c].g, kz);
+  a.kz = kz;
+  if (grid > resident_blocks<NS>(h8_cheb_batch_kernel<NS>, kz)) return PHASTB_UNSUPPORTED;
+  return launch<NS>(h8_cheb_batch_kernel<NS>, a, (int)grid, s);
+}
+
+}  // namespace
+
+size_t coarse_cheb_bytes(long long nodes) {
+  return align_up(2 * sizeof(Tagged) * (size_t)nodes) + align_up(sizeof(unsigned) * (kChebBlocks + 1));
+}
+
+int coarse_cheb_reset(long long nodes, void* exchange, cudaStream_t s) {
+  return cuda_status(cudaMemsetAsync(exchange, 0, coarse_cheb_bytes(nodes), s));
 }
 
 int coarse_cheb_launch(const VoxGeom& g, const float* lam, const float* mu, const float* b, const float* invd, float* x,
                        const double* bsums, double inv_theta, const double* c1, const double* c2, int steps,
                        const RedWs* sums, void* exchange, const int* guard, cudaStream_t s) {
-  int dev = 0, sms = 0, coop = 0;
   if (steps < 1 || steps > kChebMaxSteps || !persistent_pcg_enabled()) return PHASTB_UNSUPPORTED;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess) {
-    cudaGetLastError();
-    return PHASTB_UNSUPPORTED;
-  }
   ChebArgs a;
   std::memset(&a, 0, sizeof(a));
   a.tiles_x = (g.rx + OX - 1) / OX;
   a.tiles_xy = a.tiles_x * ((g.ry + OY - 1) / OY);
-  const int blocks = std::min(sms, kGridBlocks);
-  if (!coop || a.tiles_xy > blocks) return PHASTB_UNSUPPORTED;
-  // as many slabs as there are SMs for; a slab's layers go to sub-bricks first, then to their depth
-  const int slabs = std::min(blocks / a.tiles_xy, g.rz), layers = (g.rz + slabs - 1) / slabs;
-  const int ns = layers <= 1 ? 1 : (layers <= 2 ? 2 : 4);
-  a.kz = (layers + ns - 1) / ns;
-  if (a.kz > kMaxDepth) return PHASTB_UNSUPPORTED;
   a.g = g;
   a.steps = steps;
   a.k = tile_args<T>(g, 1).k;
@@ -339,11 +442,54 @@ int coarse_cheb_launch(const VoxGeom& g, const float* lam, const float* mu, cons
   a.bsums = bsums;
   if (sums) a.ws = *sums;
   a.words = static_cast<Tagged*>(exchange);
+  a.word_stride = g.n_red;
   a.epoch = reinterpret_cast<unsigned*>(static_cast<char*>(exchange) + align_up(2 * sizeof(Tagged) * (size_t)g.n_red));
-  a.err = a.epoch + kGridBlocks;
+  a.err = a.epoch + kChebBlocks;
   a.guard = guard;
-  const int grid = a.tiles_xy * ((g.rz + ns * a.kz - 1) / (ns * a.kz));
-  return ns == 1 ? launch<1>(a, grid, s) : (ns == 2 ? launch<2>(a, grid, s) : launch<4>(a, grid, s));
+  // the shallowest brick that needs no second block on an SM
+  int st = try_cell<1>(a, 1, s);
+  if (st == PHASTB_UNSUPPORTED) st = try_cell<2>(a, 1, s);
+  if (st == PHASTB_UNSUPPORTED) st = try_cell<4>(a, 1, s);
+  if (st == PHASTB_UNSUPPORTED) st = try_cell<4>(a, 2, s);
+  return st;
+}
+
+int coarse_cheb_batch_launch(const BatchCell* d_cells, const BatchCell* cells, int n_cells, long long nodes,
+                             const float* lam, const float* mu, const float* b, const float* invd, float* x,
+                             const char* bsums, const double* inv_theta, const double* inv_delta, const double* c1,
+                             const double* c2, int steps, char* sums, void* exchange, const int* guard,
+                             int guard_stride, cudaStream_t s) {
+  // (a block finds its cell by counting)
+  if (steps < 1 || steps > kChebMaxSteps || n_cells > 64 || !persistent_pcg_enabled()) return PHASTB_UNSUPPORTED;
+  ChebBatchArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.cells = d_cells;
+  a.n_cells = n_cells;
+  a.steps = steps;
+  a.guard_stride = guard_stride;
+  for (int i = 0; i < steps; ++i) {
+    a.c1[i] = c1[i];
+    a.c2[i] = c2[i];
+  }
+  a.inv_theta = inv_theta;
+  a.inv_delta = inv_delta;
+  a.lam = lam;
+  a.mu = mu;
+  a.b = b;
+  a.invd = invd;
+  a.x = x;
+  a.bsums = bsums;
+  a.sums = sums;
+  a.words = static_cast<Tagged*>(exchange);
+  a.word_stride = nodes;
+  a.epoch = reinterpret_cast<unsigned*>(static_cast<char*>(exchange) + align_up(2 * sizeof(Tagged) * (size_t)nodes));
+  a.err = a.epoch + kChebBlocks;
+  a.guard = guard;
+  int st = try_batch<1>(a, cells, 1, s);
+  if (st == PHASTB_UNSUPPORTED) st = try_batch<2>(a, cells, 1, s);
+  if (st == PHASTB_UNSUPPORTED) st = try_batch<4>(a, cells, 1, s);
+  if (st == PHASTB_UNSUPPORTED) st = try_batch<4>(a, cells, 2, s);
+  return st;
 }
 
 }  // namespace phastb
