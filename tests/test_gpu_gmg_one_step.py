@@ -42,3 +42,21 @@ def test_one_step_cycle(shape, periodic, mixed, levels, free_strain):
     act = op.mech_operator(d=d)
     assert info.converged and bool((x[mask] == values[mask]).all())
     assert float(act(x)[~mask].norm()) <= 2 * RTOL * float(act(values)[~mask].norm())
+
+
+@pytest.mark.parametrize("sizes,n", [((32,), 1), ((32, 36, 48), 5), ((96,), 3)])
+def test_one_step_cycle_batched(sizes, n):
+    """One cell, cells of several sizes in one launch, and cells too many for bricks of one layer."""
+    from test_gpu_batch_packed import _setup
+    from phast_b200 import solid3d as s3
+    cells, load, ops, B = _setup(sizes=sizes, n=n, brick=(8, 8, 8))
+    rng = np.random.default_rng(23)
+    ds = [torch.as_tensor(rng.uniform(0.0, 0.6, op.n_red), device="cuda") for op in ops]
+    values = [op.mech_fixed_values(0.004 + 0.001 * c) for c, op in enumerate(ops)]
+    form = s3.MechForm("gmg", mixed=True, smooth_degree=1, coarse_degree=6, inner_rtol=1e-5)
+    x, status, its, conv, bn, rn = B.mech_solve(B.pack_nodes(ds), B.pack_mech(values), rtol=RTOL, mixed=True,
+                                                form=form, reuse_lmax=False)
+    assert status == 0 and conv.all()
+    for c, op in enumerate(ops):
+        act, free, xc = op.mech_operator(d=ds[c]), ~op.mech_fixed_mask(), B.mech_view(x, c)
+        assert float(act(xc)[free].norm()) <= 2 * RTOL * float(act(values[c])[free].norm())
