@@ -49,7 +49,7 @@ def test_one_step_cycle_batched(sizes, n):
     """One cell, cells of several sizes in one launch, and cells too many for bricks of one layer."""
     from test_gpu_batch_packed import _setup
     from phast_b200 import solid3d as s3
-    cells, load, ops, B = _setup(sizes=sizes, n=n, brick=(8, 8, 8))
+    cells, load, ops, B = _setup(sizes=sizes, n=n, brick=(16, 8, 8))
     rng = np.random.default_rng(23)
     ds = [torch.as_tensor(rng.uniform(0.0, 0.6, op.n_red), device="cuda") for op in ops]
     values = [op.mech_fixed_values(0.004 + 0.001 * c) for c, op in enumerate(ops)]
