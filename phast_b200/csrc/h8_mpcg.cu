@@ -5,7 +5,9 @@
 // owned nodes live in shared memory, and per iteration only the neighbours' z on the brick's rim (tagged words) and
 // the two reductions cross the chip (grid_sync.cuh).  What bounds it: the latency of the march, with eight warps of
 // up to 255 registers per SM, and the two waits on the grid.  As separate launches (action 10 us, update 7, direction
-// 2, and the gaps) a 32^3 iteration took 21 us; here it takes 11.5.
+// 2, and the gaps) a 32^3 iteration took 21 us; here it takes 11.5.  Whole solves, separate launches and this: 12^3 3.9 / 2.0
+// ms, 24^3 8.7 / 4.6, 32^3 12.8 / 7.6, 40^3 20.2 / 12.8, 48^3 28.0 / 20.9 (about the largest that fits).  Four
+// sub-bricks of 96 threads at 168 registers: 8.0 ms at 32^3 and 35 at 48^3, from the spills and the repeated layers.
 #include <algorithm>
 #include <cstring>
 
