@@ -709,6 +709,17 @@ int phastb_h8_tma_staging(const phastb_voxel_grid* g, int dtype);
 int phastb_test_grid_barrier(int blocks, int skip_block, double limit_s, int* grid_error_host,
                              int* passed_host);
 
+/* Self-test of the exchange words that the one-launch solves wait on (no counterpart in the
+ * reference).  `blocks` (at most 148) blocks of a cooperative launch take three steps, each a word
+ * from the next block and a sum over the grid, and block 0 stores the solve's state at the end.
+ * failure 0: none; 1: in the second step block `who` leaves before it sends its word; 2: before it
+ * adds to the sum; 3: it reports that a wait of its own ran out and goes on.  A wait ends after
+ * limit_s seconds (at most 10) of GPU time.  Returns PHASTB_ERR_CUDA with *grid_error_host = 1
+ * when a failure was reported, PHASTB_OK with 0 otherwise; *passed_host counts the blocks that got
+ * through with the right values. */
+int phastb_test_grid_exchange(int blocks, int who, int failure, double limit_s, int* grid_error_host,
+                              int* passed_host);
+
 /* ---- Packed batches of periodic voxel cells --------------------------------------------
  * PhAST runs one cell per Problem.run (solid3d/api.py:191-233); these entry points advance
  * many cells of different sizes together.  A batch plan fixes the cells' grids, phase-field

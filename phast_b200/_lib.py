@@ -179,6 +179,7 @@ SIGNATURES = {
     "phastb_h8_damage_residual_norm": (C.c_int, [VG, VM, vp, vp, C.c_double, vp, dp, vp, sz, vp]),
     "phastb_scale_set": (C.c_int, [C.c_int, vp, C.c_double, C.c_int, C.c_double, vp, vp]),
     "phastb_test_grid_barrier": (C.c_int, [C.c_int, C.c_int, C.c_double, ip, ip]),
+    "phastb_test_grid_exchange": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_double, ip, ip]),
     "phastb_h8_tma_staging": (C.c_int, [VG, C.c_int]),
     "phastb_batch_create": (vp, [C.c_int, VG, dp, dp, C.c_int, C.c_int, C.c_int]),
     "phastb_batch_destroy": (None, [vp]),

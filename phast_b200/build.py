@@ -18,7 +18,7 @@ OUT_DIR = os.path.join(HERE, "_lib")
 LIB = os.path.join(OUT_DIR, "libphastb.so")
 SOURCES = ["capi.cu", "q4.cu", "h8.cu", "h8_tile.cu", "h8_dpcg.cu", "h8_mpcg.cu", "h8_cheb.cu", "engine.cu",
            "solvers2d.cu", "q4_krylov.cu", "solvers3d.cu", "gmg.cu", "t3.cu", "t3_krylov.cu", "batch3d.cu", "pfczm.cu",
-           "closure.cu", "anderson.cu"]
+           "closure.cu", "anderson.cu", "grid_test.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

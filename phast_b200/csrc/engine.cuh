@@ -88,6 +88,21 @@ struct PcgState {
   int pad_;
 };
 
+// What the one writing block of a persistent kernel leaves of its copy S of the state.  Not grid_error: another block
+// may have set it since S was read, and nothing may take that back.
+__device__ __forceinline__ void store_pcg_state(PcgState* st, const PcgState& S) {
+  st->rz = S.rz;
+  st->rr = S.rr;
+  st->alpha = S.alpha;
+  st->beta = S.beta;
+  st->active = S.active;
+  st->breakdown = S.breakdown;
+  st->nonfinite = S.nonfinite;
+  st->steps = S.steps;
+  st->iter = S.iter;
+  st->converged = S.converged;
+}
+
 // PcgState::grid_error of a persistent kernel that left the solve untouched (a form it does not have).
 constexpr int kGridDeclined = 2;
 

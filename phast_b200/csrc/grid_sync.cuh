@@ -43,7 +43,8 @@ __device__ __forceinline__ Tagged ld_tagged(const Tagged* p) {
 }
 
 // Waits (bounded) until p carries `tag`; its value through *v.  False: gave up, or another wait of the grid has.
-__device__ __forceinline__ bool wait_tagged(const Tagged* p, unsigned long long tag, double* v, unsigned* err) {
+__device__ __forceinline__ bool wait_tagged(const Tagged* p, unsigned long long tag, double* v, unsigned* err,
+                                            unsigned long long limit_ns = kGridLimitNs) {
   Tagged t = ld_tagged(p);
   if (t.tag != tag) {
     const unsigned long long t0 = grid_clock_ns();
@@ -51,13 +52,40 @@ __device__ __forceinline__ bool wait_tagged(const Tagged* p, unsigned long long 
       t = ld_tagged(p);
       if (t.tag == tag) break;
       if ((i & 255u) == 0u && (*reinterpret_cast<volatile unsigned*>(err) != 0u || i >= kGridPolls ||
-                               grid_clock_ns() - t0 > kGridLimitNs)) {
+                               grid_clock_ns() - t0 > limit_ns)) {
         atomicExch(err, 1u);
         return false;
       }
     }
   }
   *v = t.v;
+  return true;
+}
+
+// Three single-precision values and the step they belong to in one 16-byte word.
+__device__ __forceinline__ void st_node(Tagged* p, float x, float y, float z, unsigned tag) {
+  st_tagged(p, __hiloint2double(__float_as_int(y), __float_as_int(x)),
+            ((unsigned long long)tag << 32) | (unsigned)__float_as_int(z));
+}
+// Waits (bounded) for the word of step `tag`; false: gave up, or another wait of the grid has.
+__device__ __forceinline__ bool wait_node(const Tagged* p, unsigned tag, float (&v)[3], unsigned* err,
+                                          unsigned long long limit_ns = kGridLimitNs) {
+  Tagged t = ld_tagged(p);
+  if ((unsigned)(t.tag >> 32) != tag) {
+    const unsigned long long t0 = grid_clock_ns();
+    for (unsigned i = 1;; ++i) {
+      t = ld_tagged(p);
+      if ((unsigned)(t.tag >> 32) == tag) break;
+      if ((i & 255u) == 0u && (*reinterpret_cast<volatile unsigned*>(err) != 0u || i >= kGridPolls ||
+                               grid_clock_ns() - t0 > limit_ns)) {
+        atomicExch(err, 1u);
+        return false;
+      }
+    }
+  }
+  v[0] = __int_as_float(__double2loint(t.v));
+  v[1] = __int_as_float(__double2hiint(t.v));
+  v[2] = __int_as_float((int)(unsigned)t.tag);
   return true;
 }
 
@@ -77,6 +105,7 @@ struct GridSync {
   Tagged* slots;
   unsigned* err;
   unsigned long long phase;  // reductions done, the same in every thread of the grid
+  unsigned long long limit_ns = kGridLimitNs;  // of one wait
 };
 
 // Sums of v[0..K) and minima of v[K..K+M) over every thread of the grid, in every thread, in an order fixed by
@@ -120,11 +149,11 @@ __device__ __forceinline__ bool grid_reduce(double (&v)[K + M], GridSync& g, Ove
       if (l == 0) st_tagged(in + (size_t)w * G + blockIdx.x, t, tag);
       if (direct) {
         t = sum ? 0.0 : INFINITY;
-        if (l < G && !wait_tagged(in + (size_t)w * G + l, tag, &t, g.err)) s_bad = 1;
+        if (l < G && !wait_tagged(in + (size_t)w * G + l, tag, &t, g.err, g.limit_ns)) s_bad = 1;
         t = fold(sum, t);
         if (l == 0) s_out[w] = t;
       } else if (!root) {
-        if (l == 0 && !wait_tagged(res + (size_t)w * G + blockIdx.x, tag, &s_out[w], g.err)) s_bad = 1;
+        if (l == 0 && !wait_tagged(res + (size_t)w * G + blockIdx.x, tag, &s_out[w], g.err, g.limit_ns)) s_bad = 1;
       }
     }
   }
@@ -135,7 +164,7 @@ __device__ __forceinline__ bool grid_reduce(double (&v)[K + M], GridSync& g, Ove
       const bool sum = k < K;
       const int b = 32 * part + l;
       double t = sum ? 0.0 : INFINITY;
-      if (b < G && !wait_tagged(in + (size_t)k * G + b, tag, &t, g.err)) s_bad = 1;
+      if (b < G && !wait_tagged(in + (size_t)k * G + b, tag, &t, g.err, g.limit_ns)) s_bad = 1;
       t = fold(sum, t);
       if (l == 0) s_fold[k][part] = t;
     }

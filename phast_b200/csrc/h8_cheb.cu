@@ -79,32 +79,6 @@ struct ChebLayout {
   }
 };
 
-// A node's three values and the step they belong to in one 16-byte word.
-__device__ __forceinline__ void st_node(Tagged* p, T x, T y, T z, unsigned tag) {
-  st_tagged(p, __hiloint2double(__float_as_int(y), __float_as_int(x)),
-            ((unsigned long long)tag << 32) | (unsigned)__float_as_int(z));
-}
-// Waits (bounded) for the word of step `tag`; false: gave up, or another wait of the grid has.
-__device__ __forceinline__ bool wait_node(const Tagged* p, unsigned tag, T (&v)[3], unsigned* err) {
-  Tagged t = ld_tagged(p);
-  if ((unsigned)(t.tag >> 32) != tag) {
-    const unsigned long long t0 = grid_clock_ns();
-    for (unsigned i = 1;; ++i) {
-      t = ld_tagged(p);
-      if ((unsigned)(t.tag >> 32) == tag) break;
-      if ((i & 255u) == 0u && (*reinterpret_cast<volatile unsigned*>(err) != 0u || i >= kGridPolls ||
-                               grid_clock_ns() - t0 > kGridLimitNs)) {
-        atomicExch(err, 1u);
-        return false;
-      }
-    }
-  }
-  v[0] = __int_as_float(__double2loint(t.v));
-  v[1] = __int_as_float(__double2hiint(t.v));
-  v[2] = __int_as_float((int)(unsigned)t.tag);
-  return true;
-}
-
 // Brick vb of the vgrid bricks of one grid.
 template <int NS>
 __device__ __forceinline__ void cheb_body(const ChebArgs& a, int vb, int vgrid) {

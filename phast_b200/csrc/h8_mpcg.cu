@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(kT, 1) h8_mpcg_kernel(MBrickArgs a, VoxMat<T> 
       }
     }
   }
-  if (blockIdx.x == 0 && tid == 0) *a.st = S;
+  if (blockIdx.x == 0 && tid == 0) store_pcg_state(a.st, S);
 }
 
 // Bricks of one shape: the least depth that covers the grid with at most `blocks` blocks; 0 when none fits.

@@ -1006,19 +1006,7 @@ __global__ void __launch_bounds__(kTileMaxThreads, 2) h8_damage_pcg_kernel(DTile
       }
       if (S.breakdown || S.nonfinite) S.active = 0;
     }
-    if (blockIdx.x == 0 && tid == 0) {
-      PcgState& o = *c.st;
-      o.rz = S.rz;
-      o.rr = S.rr;
-      o.alpha = S.alpha;
-      o.beta = S.beta;
-      o.active = S.active;
-      o.breakdown = S.breakdown;
-      o.nonfinite = S.nonfinite;
-      o.steps = S.steps;
-      o.iter = S.iter;
-      o.converged = S.converged;
-    }
+    if (blockIdx.x == 0 && tid == 0) store_pcg_state(c.st, S);
     const T* t = p_src;
     p_src = p_dst;
     p_dst = const_cast<T*>(t);

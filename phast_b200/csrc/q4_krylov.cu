@@ -447,7 +447,7 @@ __global__ void __launch_bounds__(kT, 1) q4_pcg_kernel(ROWS rows, PcgArgs a) {
       }
     }
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) *a.st = S;
+  if (blockIdx.x == 0 && threadIdx.x == 0) store_pcg_state(a.st, S);
 }
 
 // ------------------------------------------------------------------ PPCG
