@@ -14,7 +14,9 @@
  *   - `dtype` selects the storage/arithmetic type of the vectors: PHASTB_F64 or
  *     PHASTB_F32.  Inner products, norms and reductions are always FP64.
  *   - Scratch memory comes from a caller-provided workspace whose size is given
- *     by the matching *_workspace_bytes function.
+ *     by the matching *_workspace_bytes function.  A workspace aligned to 16 bytes
+ *     lets the solvers take their one-launch forms; one aligned to 8 bytes is served
+ *     by separate launches.
  *
  * Each declaration cites the PhAST function (src/phast/..., file:line) whose
  * behaviour it reproduces.

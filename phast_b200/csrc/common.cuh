@@ -168,7 +168,9 @@ __device__ __forceinline__ int fold_or(const int* part, int n, int* sh) {
 
 template <typename T> __device__ __forceinline__ T ld(const T* p) { return __ldg(p); }
 
-__device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+__host__ __device__ __forceinline__ bool aligned16(const void* p) {
+  return (reinterpret_cast<uintptr_t>(p) & 15u) == 0;
+}
 
 // The 16-byte vector of a word type.
 template <typename T>

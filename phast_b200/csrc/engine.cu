@@ -746,7 +746,8 @@ __global__ void __launch_bounds__(kThreads) pcg_update_dot_kernel(int n, PcgWs<T
     constexpr int V = 16 / sizeof(T);
     using Vec = typename Vec16<T>::type;
     int tail = 0;
-    if (aligned16(x) && (!inv_diag || aligned16(inv_diag))) {
+    // (the workspace's vectors lie at multiples of 256 bytes from one base)
+    if (aligned16(x) && aligned16(w.r) && (!inv_diag || aligned16(inv_diag))) {
       tail = n / V * V;
       for (int c = t0; c < n / V; c += step) {
         T xv[V], pv[V], rv[V], av[V], dv[V], zv[V];

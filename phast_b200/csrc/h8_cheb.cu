@@ -396,7 +396,7 @@ int coarse_cheb_reset(long long nodes, void* exchange, cudaStream_t s) {
 int coarse_cheb_launch(const VoxGeom& g, const float* lam, const float* mu, const float* b, const float* invd, float* x,
                        const double* bsums, double inv_theta, const double* c1, const double* c2, int steps,
                        const RedWs* sums, void* exchange, const int* guard, cudaStream_t s) {
-  if (steps < 1 || steps > kChebMaxSteps || !persistent_pcg_enabled()) return PHASTB_UNSUPPORTED;
+  if (steps < 1 || steps > kChebMaxSteps || !aligned16(exchange) || !persistent_pcg_enabled()) return PHASTB_UNSUPPORTED;
   ChebArgs a;
   std::memset(&a, 0, sizeof(a));
   a.tiles_x = (g.rx + OX - 1) / OX;
@@ -435,7 +435,8 @@ int coarse_cheb_batch_launch(const BatchCell* d_cells, const BatchCell* cells, i
                              const double* c2, int steps, char* sums, void* exchange, const int* guard,
                              int guard_stride, cudaStream_t s) {
   // (a block finds its cell by counting)
-  if (steps < 1 || steps > kChebMaxSteps || n_cells > 64 || !persistent_pcg_enabled()) return PHASTB_UNSUPPORTED;
+  if (steps < 1 || steps > kChebMaxSteps || n_cells > 64 || !aligned16(exchange) || !persistent_pcg_enabled())
+    return PHASTB_UNSUPPORTED;
   ChebBatchArgs a;
   std::memset(&a, 0, sizeof(a));
   a.cells = d_cells;

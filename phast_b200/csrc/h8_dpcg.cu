@@ -366,7 +366,8 @@ int h8_damage_brick_pcg(const DTileArgs<T>& d, const PcgWs<T>& w, void* tagged, 
     cudaGetLastError();
     return PHASTB_UNSUPPORTED;
   }
-  if (!coop || !tagged || mode == PCG_PERIODIC || !persistent_pcg_enabled()) return PHASTB_UNSUPPORTED;
+  if (!coop || !tagged || !aligned16(tagged) || !aligned16(w.part) || mode == PCG_PERIODIC || !persistent_pcg_enabled())
+    return PHASTB_UNSUPPORTED;
   const int blocks = std::min(sms, kGridBlocks);
   // 16 x 14 bricks recompute the least halo; 14 x 7 and 8 x 8 follow ragged grids more closely.  The march is
   // kz + 1 layers whatever the shape, so the least depth wins.

@@ -397,7 +397,7 @@ int h8_mech_brick_pcg(const VoxGeom& g, const VoxMat<double>& m, const uint8_t* 
   }
   const size_t words = 3 * (size_t)g.n_red;
   if (!coop || mode == PCG_PERIODIC || !mask || tagged_bytes < words * sizeof(Tagged) ||
-      (reinterpret_cast<uintptr_t>(tagged) & 15u) || !persistent_pcg_enabled())
+      !aligned16(tagged) || !aligned16(w.part) || !persistent_pcg_enabled())
     return PHASTB_UNSUPPORTED;
   const int blocks = std::min(sms, kGridBlocks);
   // the march is kz + 1 layers whatever the shape, so the least depth wins

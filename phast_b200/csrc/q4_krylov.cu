@@ -762,7 +762,7 @@ int run_pcg(const ROWS& rows, const phastb_q4_grid& grid, const PcgWs<double>& w
   a.st = w.st;
   const int nt = a.g.tx * a.g.ty;
   const size_t smem = tile_smem(a.g, ROWS::W, ROWS::NC, ROWS::NC);
-  if (smem > kSmemMax) return PHASTB_UNSUPPORTED;
+  if (smem > kSmemMax || !aligned16(a.z) || !aligned16(a.slots)) return PHASTB_UNSUPPORTED;
   int st = reset_sync(w, a.z, (size_t)ROWS::NC * a.g.NX * a.g.NY, s);
   if (st) return st;
   ROWS r = rows;
@@ -815,7 +815,7 @@ int q4_ppcg_persistent(const Q4DamageSys& sys, const PpcgWs& w, const double* d_
   a.st = w.st;
   const int nt = a.g.tx * a.g.ty;
   const size_t smem = tile_smem(a.g, DamageRows::W, 2, 1);
-  if (smem > kSmemMax) return PHASTB_UNSUPPORTED;
+  if (smem > kSmemMax || !aligned16(a.pub_z) || !aligned16(a.pub_d) || !aligned16(a.slots)) return PHASTB_UNSUPPORTED;
   const size_t n = (size_t)a.g.NX * a.g.NY;
   int st = reset_sync(w, a.pub_z, n, s);
   if (!st) st = cuda_status(cudaMemsetAsync(a.pub_d, 0, n * sizeof(Tagged), s));

@@ -28,9 +28,10 @@ struct Q4MechSys {
   const uint8_t* mask;
 };
 
-// ppcg_solve (engine.cuh) on the damage system in one launch: w.b and w.minv are formed here.
-// PHASTB_UNSUPPORTED: the grid does not fit the SMs' shared memory, or the device has no
-// cooperative launch (or PHASTB_PERSISTENT_PCG=0); nothing was launched.
+// ppcg_solve (engine.cuh) on the damage system in one launch: the right-hand side and the inverse
+// diagonal stay in registers, w.r to w.Ap carry the exchange.  PHASTB_UNSUPPORTED: the grid does not
+// fit the SMs' shared memory, the workspace is not 16-byte aligned (the exchange words are), or the
+// device has no cooperative launch (or PHASTB_PERSISTENT_PCG=0); nothing was launched.
 int q4_ppcg_persistent(const Q4DamageSys& sys, const PpcgWs& w, const double* d_prev, const double* d_init,
                        const uint8_t* fixed, const double* vals, double tol, int max_iter, int check_every, double* d,
                        int* info, cudaStream_t s);

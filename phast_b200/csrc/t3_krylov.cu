@@ -251,7 +251,8 @@ __global__ void __launch_bounds__(kT, 1) t3_ppcg_kernel(T3PpcgArgs a) {
 size_t t3_ppcg_extra_bytes(int n) { return align_up(sizeof(int) * kMaxColours * (size_t)n); }
 
 // ppcg_solve of an element-history damage model on a T3 mesh; `adj` holds t3_ppcg_extra_bytes.
-// PHASTB_UNSUPPORTED: too many nodes or colours, or no cooperative launch; nothing was launched.
+// PHASTB_UNSUPPORTED: too many nodes or colours, a workspace that is not 16-byte aligned (the exchange words are), or
+// no cooperative launch; nothing was launched.
 int t3_ppcg_persistent(const phastb_t3_mesh& mesh, const phastb_t3_damage_model& md, const double* H, const PpcgWs& w,
                        int* adj, const double* d_prev, const double* d_init, const uint8_t* fixed, const double* vals,
                        double tol, int max_iter, int check_every, double* d, int* info, cudaStream_t s) {
@@ -274,7 +275,8 @@ int t3_ppcg_persistent(const phastb_t3_mesh& mesh, const phastb_t3_damage_model&
   a.row = (a.per + 31) / 32 * 32;
   a.deg = 2 * mesh.n_colors;
   const size_t smem = (3 * sizeof(double) + sizeof(int)) * (size_t)a.deg * a.row;
-  if (!coop || a.per > kT || smem > kSmemMax) return PHASTB_UNSUPPORTED;
+  if (!coop || a.per > kT || smem > kSmemMax || !aligned16(w.r) || !aligned16(w.p) || !aligned16(w.part))
+    return PHASTB_UNSUPPORTED;
   const int grid = (n + a.per - 1) / a.per;
   a.n = n;
   a.colours = mesh.n_colors;
