@@ -93,17 +93,21 @@ namespace phastb {
 namespace {
 
 constexpr int kBatchMaxChunks = 1024;  // partials per cell and vector family (<= kMaxPartials)
+// A vector step of a cell spreads over about so many blocks before its threads take more than one entry each (eight at
+// most).  FP32 multigrid and FP64 Jacobi solves in ms, one cell of 32^3 / 40 of them: 37 blocks 15.3, 24.2 / 49.8, 204;
+// 74: 15.1, 23.1 / 49.6, 203; 148: 14.6, 21.9 / 51.8, 209; 296: 14.6, 21.9 / 54.0, 219.
+constexpr int kBatchCellBlocks = 74;
 
 void make_chunks(const std::vector<long long>& off, const std::vector<long long>& len, std::vector<BChunk>* out,
                  std::vector<int>* counts) {
   out->clear();
   counts->clear();
-  // up to eight entries per thread, fewer where the batch would leave SMs idle (about eight blocks per SM)
-  long long total = 0;
-  for (long long n : len) total += n;
-  const long long want = std::max<long long>(1, std::min<long long>(8, total / ((long long)kThreads * kMaxBlocks)));
   for (size_t c = 0; c < off.size(); ++c) {
     const long long n = len[c];
+    // The chunks set how the cell's sums are grouped, so they follow from its own length and its result does not
+    // depend on the other cells.
+    const long long want =
+        std::max<long long>(1, std::min<long long>(8, n / ((long long)kThreads * kBatchCellBlocks)));
     const long long per = (n + (long long)kThreads * kBatchMaxChunks - 1) / ((long long)kThreads * kBatchMaxChunks);
     const long long ch = (long long)kThreads * std::max(want, per);
     int j = 0;
