@@ -892,12 +892,15 @@ int pcg_run_thr(const LinOp<T>& A, int n, const PcgWs<T>& w, const T* b, const T
   const int G = grid_for(n);
   int st;
   const int custom = M != nullptr && M->apply != nullptr;
+  // Chunks of the device-side loop.  With a preconditioner it stops short of maxiter and the rest is launched one by
+  // one, so that no iteration runs beyond it; a cheap last chunk runs out instead.
+  const int trips = custom ? maxiter / check_every : (maxiter + check_every - 1) / check_every;
   if ((st = cuda_status(cudaMemsetAsync(w.counter, 0, sizeof(unsigned), s)))) return st;
   if ((st = A(x, w.Ap, nullptr, s))) return st;
   // The start-of-solve decisions (relative threshold, already converged,
   // non-finite, non-positive curvature) are taken on the device: no host
   // round trip before the first chunk.
-  { note_launch(); pcg_start_kernel<T><<<G, kThreads, 0, s>>>(n, w, b, inv_diag, custom, thr.abs * thr.abs, mode, thr.rel, thr.rel_floor, thr.outer_rr, thr.outer_thr * thr.outer_thr, (maxiter + check_every - 1) / check_every); }
+  { note_launch(); pcg_start_kernel<T><<<G, kThreads, 0, s>>>(n, w, b, inv_diag, custom, thr.abs * thr.abs, mode, thr.rel, thr.rel_floor, thr.outer_rr, thr.outer_thr * thr.outer_thr, trips); }
   if ((st = last_launch_status())) return st;
   const int* active = &w.st->active;
   if (custom) {
@@ -967,7 +970,7 @@ int pcg_run_thr(const LinOp<T>& A, int n, const PcgWs<T>& w, const T* b, const T
   // Preferred: the whole iteration loop on the device (one conditional-WHILE
   // graph, one host synchronisation per solve).  Otherwise chunks of
   // check_every iterations with a host check after each.
-  cudaGraphExec_t wexec = !looped && device_loop_enabled()
+  cudaGraphExec_t wexec = !looped && trips > 0 && device_loop_enabled()
                               ? while_graph_for(key, s, [&] { return iterate(check_every); }, active,
                                                 &w.st->trips, &w.st->max_trips, &glaunch)
                               : nullptr;
@@ -978,6 +981,12 @@ int pcg_run_thr(const LinOp<T>& A, int n, const PcgWs<T>& w, const T* b, const T
     if ((st = cuda_status(cudaMemcpyAsync(&hs, w.st, sizeof(hs), cudaMemcpyDeviceToHost, s)))) return st;
     if ((st = cuda_status(cudaStreamSynchronize(s)))) return st;
     note_launch(glaunch * (long long)hs.trips);
+    const int rest = maxiter - trips * check_every;
+    if (rest > 0 && hs.active) {
+      if ((st = iterate(rest))) return st;
+      if ((st = cuda_status(cudaMemcpyAsync(&hs, w.st, sizeof(hs), cudaMemcpyDeviceToHost, s)))) return st;
+      if ((st = cuda_status(cudaStreamSynchronize(s)))) return st;
+    }
     it = maxiter;
   } else {
     cudaGraphExec_t gexec =
