@@ -114,9 +114,15 @@ class BoundaryConditions:
 
     def _nodes_on_device(self, idx):
         """The node list on the device; indices are checked here, on the host (a device-side check aborts)."""
-        if idx.numel() and not (-self.n_nodes <= int(idx.min()) and int(idx.max()) < self.n_nodes):
+        if not isinstance(idx, torch.Tensor) or idx.dtype != torch.int64:
+            # an entry put into the list by hand may index as an array does: a sequence, a slice, a mask, one node
+            idx = torch.arange(self.n_nodes)[idx]
+        elif idx.numel() and not (-self.n_nodes <= int(idx.min()) and int(idx.max()) < self.n_nodes):
             raise IndexError(f"boundary node index out of range for {self.n_nodes} nodes")
         return idx.to(self.device)
+
+    def _value_on_device(self, value):
+        return value.to(self.device) if isinstance(value, torch.Tensor) else value
 
     # the masks are filled where they are used: the node lists are short, the nodal arrays are not (400 x 160:
     # 1.2 MB through pageable copies in every explicit step before)
@@ -126,7 +132,7 @@ class BoundaryConditions:
         for idx, c, v in self.bcs:
             where = self._nodes_on_device(idx)
             mask[where, c] = True
-            vals[where, c] = v * self.load_factor
+            vals[where, c] = self._value_on_device(v * self.load_factor)
         return mask, vals
 
     def get_pf_dirichlet_mask_values(self):
@@ -135,7 +141,7 @@ class BoundaryConditions:
         for idx, v in self.pf_dirichlet_bcs:
             where = self._nodes_on_device(idx)
             mask[where] = True
-            vals[where] = v
+            vals[where] = self._value_on_device(v)
         return mask, vals
 
 
