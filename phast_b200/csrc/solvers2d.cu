@@ -457,7 +457,9 @@ int phastb_t3_qs_solve(const phastb_t3_mesh* mesh, const phastb_q4_material* m, 
                    line_search, ls_max_steps, ls_min_alpha, ls_c, info, workspace, scope.get());
 }
 
-size_t phastb_t3_damage_linear_workspace_bytes(int n_nodes) { return phastb_q4_damage_linear_workspace_bytes(n_nodes); }
+size_t phastb_t3_damage_linear_workspace_bytes(int n_nodes) {
+  return pcg_ws_bytes<double>(n_nodes) + 2 * align_up(sizeof(double) * (size_t)n_nodes) + red_ws_bytes();
+}
 
 int phastb_t3_damage_linear_solve(const phastb_t3_mesh* mesh, const double* H, double gc_over_l0,
                                   const double* gc_over_l0_e, double gcl0, const double* gcl0_e, const double* rhs,
