@@ -917,8 +917,8 @@ int pcg_run_thr(const LinOp<T>& A, int n, const PcgWs<T>& w, const T* b, const T
     if (ls == PHASTB_OK) {
       if ((st = cuda_status(cudaMemcpyAsync(&hs, w.st, sizeof(hs), cudaMemcpyDeviceToHost, s)))) return st;
       if ((st = cuda_status(cudaStreamSynchronize(s)))) return st;
-      looped = hs.grid_error != kGridDeclined;
-      if (looped && hs.grid_error) return PHASTB_ERR_CUDA;
+      if (hs.grid_error) return PHASTB_ERR_CUDA;
+      looped = true;
     } else if (ls != PHASTB_UNSUPPORTED) {
       return ls;
     }

@@ -84,7 +84,7 @@ struct PcgState {
   int max_trips;    // ... which stops after this many (set per solve, not baked into the graph)
   // grid barrier of a persistent iteration kernel (reset by the start kernel)
   unsigned bar_count, bar_gen;
-  int grid_error;   // 1: a wait on the grid ran out, the persistent kernel stopped early; kGridDeclined
+  int grid_error;   // a wait on the grid ran out: the persistent kernel stopped early
   int pad_;
 };
 
@@ -102,9 +102,6 @@ __device__ __forceinline__ void store_pcg_state(PcgState* st, const PcgState& S)
   st->iter = S.iter;
   st->converged = S.converged;
 }
-
-// PcgState::grid_error of a persistent kernel that left the solve untouched (a form it does not have).
-constexpr int kGridDeclined = 2;
 
 template <typename T>
 struct PcgWs {

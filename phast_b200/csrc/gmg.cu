@@ -986,9 +986,15 @@ __global__ void ex_setup_kernel(int n, const uint8_t* __restrict__ fixed, const 
 }
 
 // b = where(free, rhs - image, 0) with ||b||^2
+// (n_e: so many E rows at the end; how many of them are free goes to ws.out[1])
 __global__ void __launch_bounds__(kThreads) ex_rhs_kernel(int n, const uint8_t* __restrict__ fixed,
                                                           const double* __restrict__ base, const double* image,
-                                                          double* b, RedWs ws) {
+                                                          double* b, RedWs ws, int n_e = 0) {
+  if (n_e > 0 && blockIdx.x == 0 && threadIdx.x == 0) {
+    int free_rows = 0;
+    for (int k = n - n_e; k < n; ++k) free_rows += fixed[k] ? 0 : 1;
+    ws.out[1] = free_rows;
+  }
   double acc[1] = {0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const double v = fixed[i] ? 0.0 : (base ? base[i] : 0.0) - image[i];
@@ -1136,11 +1142,11 @@ static int mech_solve_ex_impl(const phastb_voxel_grid* g, const phastb_voxel_mat
   MechOpT<double> full{v, m64, slot, dd, nullptr, L.scratch64, gg};
   MechOpT<double> freeop{v, m64, slot, dd, fixed, L.scratch64, gg};
   if ((st = mech_op_t<double>(&full, L.xc, L.r64, nullptr, s))) return st;
-  { note_launch(); ex_rhs_kernel<<<G, kThreads, 0, s>>>(n, fixed, nullptr, L.r64, L.bf, L.rw); }
+  { note_launch(); ex_rhs_kernel<<<G, kThreads, 0, s>>>(n, fixed, nullptr, L.r64, L.bf, L.rw, 6); }
   if ((st = last_launch_status())) return st;
-  double bn2;
-  if ((st = red_ws_fetch(L.rw, &bn2, 1, s))) return st;
-  const double bn = std::sqrt(bn2);
+  double rhs_out[2];  // ||b||^2 and the number of free E rows
+  if ((st = red_ws_fetch(L.rw, rhs_out, 2, s))) return st;
+  const double bn = std::sqrt(rhs_out[0]);
   if (rinfo) rinfo[0] = bn;
   if (!std::isfinite(bn)) return PHASTB_NONFINITE;
   if (bn == 0.0) {
@@ -1177,7 +1183,7 @@ static int mech_solve_ex_impl(const phastb_voxel_grid* g, const phastb_voxel_mat
                                  align_up(24 * sizeof(double) * (size_t)v.n_elem), L.x64, L.r64, mi, PCG_FREEZE, s);
       };
       if ((st = pcg_run<double>(A64, n, L.w64, L.bf, L.r64, nullptr, L.x64, thr, maxiter, check_every, PCG_FREEZE,
-                                0.0, &pr, s, &loop)))
+                                0.0, &pr, s, rhs_out[1] != 0.0 ? nullptr : &loop)))
         return st;
     }
     if ((st = cuda_status(cudaMemcpyAsync(x_out, L.x64, sizeof(double) * n, cudaMemcpyDeviceToDevice, s))))

@@ -78,16 +78,6 @@ __global__ void __launch_bounds__(kT, 1) h8_mpcg_kernel(MBrickArgs a, VoxMat<T> 
   extern __shared__ __align__(16) unsigned char smem[];
   const VoxGeom& g = a.g;
   const int tid = threadIdx.x;
-  if (a.mask) {
-    // free E rows couple every node with six more sums per iteration: left to the separate launches
-    const uint8_t* em = a.mask + 3 * (size_t)g.n_red;
-    bool all = true;
-    for (int k = 0; k < 6; ++k) all = all && em[k];
-    if (!all) {
-      if (blockIdx.x == 0 && tid == 0) a.st->grid_error = kGridDeclined;
-      return;
-    }
-  }
   const int kz = a.kz;
   const L lay(kz);
   const int PP = (NS * kz + 2) * PL;  // one component of P

@@ -231,8 +231,8 @@ template <typename T>
 int h8_damage_brick_pcg(const DTileArgs<T>& d, const PcgWs<T>& w, void* tagged, T* x, const T* inv_diag, int maxiter,
                         int mode, cudaStream_t s);
 
-// The same for the FP64 elastic operator with all six E rows masked (h8_mpcg.cu; with a free E row the kernel
-// leaves the state as it is and says so, kGridDeclined).  `tagged`: 48 bytes of scratch per node.
+// The same for the FP64 elastic operator with all six E rows masked, which the caller has to make sure of (h8_mpcg.cu).
+// `tagged`: 48 bytes of scratch per node.
 int h8_mech_brick_pcg(const VoxGeom& g, const VoxMat<double>& m, const uint8_t* slot, const double* gq,
                       const double* d, const uint8_t* mask, const PcgWs<double>& w, void* tagged,
                       size_t tagged_bytes, double* x, const double* inv_diag, int maxiter, int mode, cudaStream_t s);

@@ -126,10 +126,16 @@ __global__ void constrained_setup_kernel(int n, const uint8_t* __restrict__ fixe
 }
 
 // b_f = where(free, rhs - image, 0) with ||b_f||^2
+// (n_e: so many E rows at the end; how many of them are free goes to ws.out[1])
 __global__ void __launch_bounds__(kThreads) constrained_rhs_kernel(int n, const uint8_t* __restrict__ fixed,
                                                                    const double* __restrict__ rhs,
                                                                    const double* __restrict__ image,
-                                                                   double* __restrict__ bf, RedWs ws) {
+                                                                   double* __restrict__ bf, RedWs ws, int n_e = 0) {
+  if (n_e > 0 && blockIdx.x == 0 && threadIdx.x == 0) {
+    int free_rows = 0;
+    for (int k = n - n_e; k < n; ++k) free_rows += fixed[k] ? 0 : 1;
+    ws.out[1] = free_rows;
+  }
   double acc[1] = {0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const double v = fixed[i] ? 0.0 : (rhs ? rhs[i] : 0.0) - image[i];
@@ -366,11 +372,11 @@ static int mech_solve_impl(const phastb_voxel_grid* g, const phastb_voxel_materi
   { note_launch(); constrained_setup_kernel<<<G, kThreads, 0, s>>>(n, fixed, fixed_values, x0, xc, x_out, invd); }
   MechCtx full{v, mm, slot, gq, d, nullptr, scratch, patw, cl_ws, closure};
   if ((st = mech_op(&full, xc, w.Ap, nullptr, s))) return st;
-  { note_launch(); constrained_rhs_kernel<<<G, kThreads, 0, s>>>(n, fixed, nullptr, w.Ap, bf, rw); }
+  { note_launch(); constrained_rhs_kernel<<<G, kThreads, 0, s>>>(n, fixed, nullptr, w.Ap, bf, rw, 6); }
   if ((st = last_launch_status())) return st;
-  double bn2;
-  if ((st = red_ws_fetch(rw, &bn2, 1, s))) return st;
-  const double bn = std::sqrt(bn2);
+  double rhs_out[2];  // ||b||^2 and the number of free E rows
+  if ((st = red_ws_fetch(rw, rhs_out, 2, s))) return st;
+  const double bn = std::sqrt(rhs_out[0]);
   if (rinfo) rinfo[0] = bn;
   if (!std::isfinite(bn)) return PHASTB_NONFINITE;
   if (bn == 0.0) {
@@ -385,13 +391,14 @@ static int mech_solve_impl(const phastb_voxel_grid* g, const phastb_voxel_materi
                   closure ? nullptr : h8_apply_dot_slot(v, 8, scratch)};
   PcgResult pr{};
   if ((st = cuda_status(cudaMemcpyAsync(xw, x_out, sizeof(double) * n, cudaMemcpyDeviceToDevice, s)))) return st;
-  // small cells: all iterations in one launch, with the element scratch as its exchange words
+  // small cells under full macro-strain control: all iterations in one launch, with the element scratch as its
+  // exchange words (a free E row couples every node with six more sums per iteration)
   const PcgLoop loop = [&](int mi) {
     return h8_mech_brick_pcg(v, mm, slot, gq, d, fixed, w, scratch, align_up(24 * sizeof(double) * (size_t)v.n_elem),
                              xw, invd, mi, PCG_FREEZE, s);
   };
   if ((st = pcg_run<double>(A, n, w, bf, invd, nullptr, xw, thr, maxiter, check_every, PCG_FREEZE, 0.0, &pr, s,
-                            closure ? nullptr : &loop)))
+                            closure || rhs_out[1] != 0.0 ? nullptr : &loop)))
     return st;
   { note_launch(); where_kernel<<<G, kThreads, 0, s>>>(n, fixed, xw, xc, x_out); }
   if ((st = last_launch_status())) return st;
