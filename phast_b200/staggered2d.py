@@ -114,35 +114,43 @@ class BoundaryConditions:
 
     def _nodes_on_device(self, idx):
         """The node list on the device; indices are checked here, on the host (a device-side check aborts)."""
-        if not isinstance(idx, torch.Tensor) or idx.dtype != torch.int64:
-            # an entry put into the list by hand may index as an array does: a sequence, a slice, a mask, one node
-            idx = torch.arange(self.n_nodes)[idx]
-        elif idx.numel() and not (-self.n_nodes <= int(idx.min()) and int(idx.max()) < self.n_nodes):
+        if idx.numel() and not (-self.n_nodes <= int(idx.min()) and int(idx.max()) < self.n_nodes):
             raise IndexError(f"boundary node index out of range for {self.n_nodes} nodes")
         return idx.to(self.device)
 
-    def _value_on_device(self, value):
-        return value.to(self.device) if isinstance(value, torch.Tensor) else value
-
     # the masks are filled where they are used: the node lists are short, the nodal arrays are not (400 x 160:
-    # 1.2 MB through pageable copies in every explicit step before)
+    # 1.2 MB through pageable copies in every explicit step before).  An entry put into a list by hand may index and
+    # carry values as an array does (a sequence, a slice, a mask, one node, a value per node); a list with such an
+    # entry fills host arrays, which take and refuse exactly that
+    @staticmethod
+    def _plain(idx, value):
+        return isinstance(idx, torch.Tensor) and idx.dtype == torch.int64 and isinstance(value, (int, float))
+
     def get_masks_and_values(self):
-        mask = torch.zeros(self.n_nodes, 2, dtype=torch.bool, device=self.device)
-        vals = torch.zeros(self.n_nodes, 2, dtype=self.dtype, device=self.device)
+        on_device = all(self._plain(idx, v) and isinstance(c, int) for idx, c, v in self.bcs)
+        where = self.device if on_device else "cpu"
+        mask = torch.zeros(self.n_nodes, 2, dtype=torch.bool, device=where)
+        vals = torch.zeros(self.n_nodes, 2, dtype=self.dtype, device=where)
         for idx, c, v in self.bcs:
-            where = self._nodes_on_device(idx)
-            mask[where, c] = True
-            vals[where, c] = self._value_on_device(v * self.load_factor)
-        return mask, vals
+            i = self._nodes_on_device(idx) if on_device else _to_host(idx)
+            mask[i, c] = True
+            vals[i, c] = _to_host(v) * self.load_factor
+        return mask.to(self.device), vals.to(self.device)
 
     def get_pf_dirichlet_mask_values(self):
-        mask = torch.zeros(self.n_nodes, dtype=torch.bool, device=self.device)
-        vals = torch.zeros(self.n_nodes, dtype=self.dtype, device=self.device)
+        on_device = all(self._plain(idx, v) for idx, v in self.pf_dirichlet_bcs)
+        where = self.device if on_device else "cpu"
+        mask = torch.zeros(self.n_nodes, dtype=torch.bool, device=where)
+        vals = torch.zeros(self.n_nodes, dtype=self.dtype, device=where)
         for idx, v in self.pf_dirichlet_bcs:
-            where = self._nodes_on_device(idx)
-            mask[where] = True
-            vals[where] = self._value_on_device(v)
-        return mask, vals
+            i = self._nodes_on_device(idx) if on_device else _to_host(idx)
+            mask[i] = True
+            vals[i] = _to_host(v)
+        return mask.to(self.device), vals.to(self.device)
+
+
+def _to_host(a):
+    return a.cpu() if isinstance(a, torch.Tensor) else a
 
 
 class AndersonAccelerator:
