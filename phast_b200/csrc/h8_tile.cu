@@ -112,7 +112,7 @@ __device__ __forceinline__ void get4(const double* p, double (&v)[4]) {
 // ry, rz) array, tmd: d as (rx, ry, rz)) issued by one thread and completed on an
 // mbarrier per layer buffer; halo nodes that wrap around a periodic edge read
 // the zero fill and are patched by per-thread loads.  Otherwise every thread
-// stages its (at most two) halo-tile nodes through registers.
+// copies its (at most two) halo-tile nodes into shared memory with cp.async.
 // The action over the bricks vb, vb + vgrid, ... of one grid: a plain launch runs it with
 // its block index and grid size, a batched launch with the block's virtual index inside its cell.
 template <typename T, int COEF, int MODE, int OX, int OY, bool TMA>
@@ -1073,9 +1073,9 @@ int launch_kz(long long tiles_xy, int rz, long long capacity) {
 // Modelled time of an elastic march: `tiles` bricks of kz node layers and `warps` warps, per_sm of them resident
 // on each of `sms` SMs.  A round of resident bricks runs kz + 1 element layers plus a prologue of about one;
 // a layer costs a fixed latency (two barriers and the element's dependent chain) and issue time in proportion
-// to the warps that share a scheduler.  The coefficients (microseconds) are fitted to sweeps of shape and depth;
-// the model then gives, on 64^3, 24.6 us for FP32 16 x 8 x 5 (measured 24.6), 26.6 for 16 x 8 x 6 (26.7), 29.9
-// for 16 x 8 x 4 (28.9), and in FP64 33.1 for 16 x 14 x 10 (32.9), 42.8 for 16 x 8 x 16 (43.1).
+// to the warps that share a scheduler.  The coefficients (microseconds) come from sweeps of shape and depth and are
+// there to rank them: on 64^3 the model gives 20.8 us for FP32 16 x 8 x 5 (measured 24.6), 23.8 for 16 x 8 x 6 (26.7),
+// 29.0 for 16 x 8 x 4 (28.9), and in FP64 29.0 for 16 x 14 x 10 (32.9), 43.0 for 16 x 8 x 16 (43.1).
 double march_cost(int word, int warps, long long tiles, int per_sm, int sms, int kz) {
   const double a = word == 4 ? 0.82 : 1.5, b = word == 4 ? 0.5 : 0.42;
   const long long cap = std::min<long long>((long long)per_sm * sms, kMaxPartials);
@@ -1159,7 +1159,7 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 }
 
 // Tensor maps of u~ (a (3 rx, ry, rz) array) and d ((rx, ry, rz)) for the TMA
-// staging of a launch; false (stage through registers instead) when TMA is off,
+// staging of a launch; false (cp.async instead) when TMA is off,
 // the row strides are not multiples of 16 bytes (rx a multiple of 16 / sizeof(T)),
 // a buffer is not 16-byte aligned, or the driver refuses a map.
 template <typename T>
@@ -1407,12 +1407,6 @@ TileArgs<T> tile_args(const VoxGeom& v, int cls) {
   a.ts = clamp_shape(tile_shape_for(v, (int)sizeof(T), cls), v);
   a.k.c1 = T(kC1);
   a.k.c2 = T(kC2);
-  a.k.x1 = T(kC1 / v.hx);
-  a.k.x2 = T(kC2 / v.hx);
-  a.k.y1 = T(kC1 / v.hy);
-  a.k.y2 = T(kC2 / v.hy);
-  a.k.z1 = T(kC1 / v.hz);
-  a.k.z2 = T(kC2 / v.hz);
   set_modal_k(a.k, v);
   return a;
 }
@@ -1583,7 +1577,6 @@ int h8_damage_tile_launch(const VoxGeom& v, const VoxMat<T>& m, const uint8_t* s
   const TileArgs<T> base = tile_args<T>(v, 2);
   a.g = v;
   a.ts = base.ts;
-  a.k = base.k;
   a.slot = slot;
   a.kappa = double(m.kappa);
   a.ell = double(m.ell);
@@ -1661,7 +1654,6 @@ int h8_damage_pcg_launch(const VoxGeom& v, const VoxMat<T>& m, const uint8_t* sl
   const TileArgs<T> base = tile_args<T>(v, 2);
   a.g = v;
   a.ts = base.ts;
-  a.k = base.k;
   a.slot = slot;
   a.kappa = double(m.kappa);
   a.ell = double(m.ell);
@@ -1777,7 +1769,6 @@ __global__ void __launch_bounds__(kTileMaxThreads, 2) h8_dtile_batch_kernel(Tile
     a.mask = b.mask ? b.mask + c.node_off : nullptr;
     a.ws = red_ws(b.ws + (size_t)wk.x * red_ws_bytes());
     a.guard = b.guard ? b.guard + (size_t)wk.x * b.guard_stride : nullptr;
-    a.k = batch_k<T>(c);
     sa = a;
   }
   __syncthreads();

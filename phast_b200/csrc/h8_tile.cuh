@@ -128,12 +128,10 @@ enum TileMode {
   kModeApply = 0, kModeDot = 1, kModeEnergy = 2, kModeCheb = 3, kModeNodal = 4, kModeRes = 5, kModeSmooth = 6
 };
 
-// Gauss-point constants of the action: N1 weights with the 1/h of each axis
-// folded in (the last interpolation stage of a derivative applies them).
+// Constants of the action: interpolation weights of the Gauss points and the scales of the modal form.
 template <typename T>
 struct TileK {
-  T c1, c2;                  // N1 = [[c1, c2], [c2, c1]]
-  T x1, x2, y1, y2, z1, z2;  // c1/h, c2/h per axis
+  T c1, c2;  // N1 = [[c1, c2], [c2, c1]]
   // modal form: g = 1/sqrt(3) (the Gauss coordinate), and per axis a = 1/(4 h), b = a g
   T g, ax, ay, az, bx, by, bz;
 };
@@ -200,7 +198,6 @@ struct DTileArgs {
   const uint8_t* mask;
   RedWs ws;
   const int* guard;
-  TileK<T> k;
 };
 
 // Damage action y = scale [Gc (M/ell + ell L) + 2 (1-kappa) H-mass] x on the
