@@ -16,9 +16,6 @@ namespace phastb {
 constexpr int kThreads = 256;        // block size of every vector/reduction kernel
 constexpr int kMaxBlocks = 148 * 8;  // 8 resident blocks per SM on 148 SMs
 constexpr int kMaxPartials = kMaxBlocks;
-// Blocks of a vector kernel that ends in a sum over the grid: the arrivals queue on one counter (a CG update of
-// 786 432 values: 7.1 us with 1184 blocks, 5.0 with 296, 2.5 without the sum).
-constexpr int kReduceBlocks = 148 * 2;
 
 inline int grid_for(long long n, int threads = kThreads) {
   long long b = (n + threads - 1) / threads;

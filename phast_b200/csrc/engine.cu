@@ -870,6 +870,16 @@ __global__ void __launch_bounds__(kThreads) pcg_dir_rz_kernel(int n, PcgWs<T> w,
   }
 }
 
+// Blocks of the fused CG update.  It ends in a sum over the grid whose arrivals queue on one counter (786 432 FP32
+// values: 7.1 us with 1184 blocks, 5.0 with 296, 2.5 without the sum), and the long vectors of a large cell need blocks
+// enough to keep HBM busy.  Solves with 296 / 444 / 592 / 1184 blocks in ms, FP64: 64^3 2.12, 2.10, 2.11, 2.26; 128^3
+// 29.4, 28.6, 28.6, 28.6; 192^3 134.4, 130.7, 132.0, 131.9.  FP32 multigrid: 64^3 9.53, 9.53, 9.70, 9.81.  FP32: 64^3
+// 4.24, 4.23, 4.21, 4.54; 128^3 45.2, 43.6, 42.8, 43.2; 192^3 201, 194, 191, 193.
+template <typename T>
+int update_blocks(int n) {
+  return std::min(grid_for(n), sizeof(T) == 4 && n > (1 << 21) ? 148 * 4 : 148 * 3);
+}
+
 template <typename T>
 int pcg_run(const LinOp<T>& A, int n, const PcgWs<T>& w, const T* b, const T* inv_diag, const Precond<T>* M, T* x,
             double thr, int maxiter, int check_every, PcgMode mode, double, PcgResult* out, cudaStream_t s,
@@ -928,7 +938,7 @@ int pcg_run_thr(const LinOp<T>& A, int n, const PcgWs<T>& w, const T* b, const T
     for (int k = 0; k < k_iters; ++k) {
       if (A.apply_dot) {
         if ((e = A.apply_dot(A.ctx, w.p, w.Ap, active, s))) return e;
-        { note_launch(); pcg_update_dot_kernel<T><<<std::min(G, kReduceBlocks), kThreads, 0, s>>>(n, w, x, inv_diag, custom, mode, check_every, A.dot_out); }
+        { note_launch(); pcg_update_dot_kernel<T><<<update_blocks<T>(n), kThreads, 0, s>>>(n, w, x, inv_diag, custom, mode, check_every, A.dot_out); }
       } else {
         if ((e = A(w.p, w.Ap, active, s))) return e;
         { note_launch(); pcg_alpha_kernel<T><<<G, kThreads, 0, s>>>(n, w, mode); }
