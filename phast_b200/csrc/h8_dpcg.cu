@@ -231,6 +231,8 @@ __global__ void __launch_bounds__(kT, 1) h8_dpcg_kernel(BrickArgs<T> a) {
           // two corner buffers in turn: a buffer is written again after the next layer's barrier
           sub_barrier(1 + sub, TPS);
           if (owner) {
+            // (diagonal pairs first; h8_dtile_kernel adds the four in rows.  Either rounds alike, but the last
+            // places move iteration counts of several hundred by a few, which the fixtures' tests compare exactly.)
             T v = (fc[f0] + fc[f3]) + (fc[f1] + fc[f2]);
             if (masked >> (kk - 1) & 1u) v = T(0);
             *ao = v;
