@@ -97,9 +97,14 @@ constexpr int kBatchMaxChunks = 1024;  // partials per cell and vector family (<
 // most).  FP32 multigrid and FP64 Jacobi solves in ms, one cell of 32^3 / 40 of them: 37 blocks 15.3, 24.2 / 49.8, 204;
 // 74: 15.1, 23.1 / 49.6, 203; 148: 14.6, 21.9 / 51.8, 209; 296: 14.6, 21.9 / 54.0, 219.
 constexpr int kBatchCellBlocks = 74;
+// The same over the nodes of the cells themselves, where the damage CG's two sums an iteration queue on a counter per
+// cell.  Damage solves in ms with 74 / 50 / 37 blocks: one 32^3 cell 4.40, 4.46, 4.52, four of 32^3 to 64^3 8.11, 8.13,
+// 8.16, sixteen 22.6, 21.7, 21.8, seventy of 32^3 29.4, 27.5, 27.0.  (The coarse levels' transfers lose by longer ones:
+// a mechanics solve of the four cells 23.9 ms, 25.0 with 37 blocks there too.)
+constexpr int kBatchNodeBlocks = 50;
 
-void make_chunks(const std::vector<long long>& off, const std::vector<long long>& len, std::vector<BChunk>* out,
-                 std::vector<int>* counts) {
+void make_chunks(const std::vector<long long>& off, const std::vector<long long>& len, int cell_blocks,
+                 std::vector<BChunk>* out, std::vector<int>* counts) {
   out->clear();
   counts->clear();
   for (size_t c = 0; c < off.size(); ++c) {
@@ -107,7 +112,7 @@ void make_chunks(const std::vector<long long>& off, const std::vector<long long>
     // The chunks set how the cell's sums are grouped, so they follow from its own length and its result does not
     // depend on the other cells.
     const long long want =
-        std::max<long long>(1, std::min<long long>(8, n / ((long long)kThreads * kBatchCellBlocks)));
+        std::max<long long>(1, std::min<long long>(8, n / ((long long)kThreads * cell_blocks)));
     const long long per = (n + (long long)kThreads * kBatchMaxChunks - 1) / ((long long)kThreads * kBatchMaxChunks);
     const long long ch = (long long)kThreads * std::max(want, per);
     int j = 0;
@@ -1767,8 +1772,9 @@ GraphKey mech_key(const phastb_batch* B, const void* mat, size_t mat_bytes, cons
 
 extern "C" {
 
-phastb_batch* phastb_batch_create(int n_cells, const phastb_voxel_grid* grids, const double* ell,
-                                  const double* dscale, int ox, int oy, int kz) {
+// A plan of the cells and, where they allow it, of their coarse multigrid levels (node_blocks: see make_chunks).
+static phastb_batch* batch_plan(int n_cells, const phastb_voxel_grid* grids, const double* ell, const double* dscale,
+                                int ox, int oy, int kz, int node_blocks) {
   if (n_cells < 1 || !grids || !ell || !dscale) return nullptr;
   if (!((ox == 16 && oy == 8) || (ox == 8 && oy == 8)) || kz < 1) return nullptr;
   phastb_batch* B = new phastb_batch();
@@ -1824,8 +1830,8 @@ phastb_batch* phastb_batch_create(int n_cells, const phastb_voxel_grid* grids, c
                    [&](int a, int b) { return B->cells[a].nvb > B->cells[b].nvb; });
   for (int c : order)
     for (int t = 0; t < B->cells[c].nvb; ++t) B->work.push_back(make_int2(c, t));
-  make_chunks(noff, nlen, &B->node_chunks, &B->node_nchunk);
-  make_chunks(moff, mlen, &B->mech_chunks, &B->mech_nchunk);
+  make_chunks(noff, nlen, node_blocks, &B->node_chunks, &B->node_nchunk);
+  make_chunks(moff, mlen, kBatchCellBlocks, &B->mech_chunks, &B->mech_nchunk);
   size_t t = 0;
   t += align_up(sizeof(BatchCell) * B->cells.size());
   t += align_up(sizeof(int2) * B->work.size());
@@ -1851,7 +1857,7 @@ phastb_batch* phastb_batch_create(int n_cells, const phastb_voxel_grid* grids, c
         g.hy *= 2;
         g.hz *= 2;
       }
-      B->lev[l] = phastb_batch_create(n_cells, cg.data(), ell, dscale, 8, 8, 4);
+      B->lev[l] = batch_plan(n_cells, cg.data(), ell, dscale, 8, 8, 4, kBatchCellBlocks);
       gmg = B->lev[l] != nullptr;
     }
     if (gmg) {
@@ -1870,6 +1876,11 @@ phastb_batch* phastb_batch_create(int n_cells, const phastb_voxel_grid* grids, c
     }
   }
   return B;
+}
+
+phastb_batch* phastb_batch_create(int n_cells, const phastb_voxel_grid* grids, const double* ell,
+                                  const double* dscale, int ox, int oy, int kz) {
+  return batch_plan(n_cells, grids, ell, dscale, ox, oy, kz, kBatchNodeBlocks);
 }
 
 void phastb_batch_destroy(phastb_batch* B) { delete B; }
